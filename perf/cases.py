@@ -11,7 +11,8 @@ A case is one pass of one of five kinds:
 
 Head dimension 128 and bf16 are all the library has.  ``listed()`` gives one case for each kind of use,
 ``draw()`` more of the same ranges, ``prepare()`` / ``run()`` execute one, ``work()`` counts the bytes and
-operations it cannot do without and ``tolerance()`` says how far two correct results may be apart.
+operations it cannot do without, ``tolerance()`` says how far two correct results may be apart and ``exact()``
+gives the same attention in 64 bits.
 """
 from __future__ import annotations
 
@@ -206,3 +207,53 @@ def tolerance(case):
     # bf16 results), and one value by at most 0.13 of the root mean square (dq of a causal sequence's first rows, whose
     # terms are many times the mean): four times that.
     return {"rel": 1e-2, "max": 0.5}
+
+
+def _attend(q, k, v, dout, causal):
+    """One sequence in 64 bits: q, dout [sq, QH, 128], k, v [sk, KVH, 128] -> out, lse [QH, sq], dq, dk, dv."""
+    sq, sk, qh, group = q.size(0), k.size(0), q.size(1), q.size(1) // k.size(1)
+    scale = 1.0 / math.sqrt(HEAD_DIM)
+    out, lse = torch.empty_like(q), q.new_empty((qh, sq))
+    dq, dk, dv = torch.zeros_like(q), torch.zeros_like(k), torch.zeros_like(v)
+    for r0 in range(0, sq, 2048):
+        r1 = min(r0 + 2048, sq)
+        seen = min(sk, r1 + sk - sq) if causal else sk
+        hidden = None
+        if causal:
+            hidden = (torch.arange(seen, device=q.device)[None, :]
+                      > torch.arange(r0, r1, device=q.device)[:, None] + (sk - sq))
+        for h in range(qh):
+            kh, vh = k[:seen, h // group], v[:seen, h // group]
+            s = (q[r0:r1, h] @ kh.T).mul_(scale)
+            if hidden is not None:
+                s.masked_fill_(hidden, -math.inf)
+            lse[h, r0:r1] = torch.logsumexp(s, dim=1)
+            p = s.sub_(lse[h, r0:r1, None]).exp_()
+            out[r0:r1, h] = p @ vh
+            if dout is not None:
+                do = dout[r0:r1, h]
+                dv[:seen, h // group] += p.T @ do
+                ds = (do @ vh.T).sub_((do * out[r0:r1, h]).sum(1, keepdim=True)).mul_(p).mul_(scale)
+                dq[r0:r1, h] = ds @ kh
+                dk[:seen, h // group] += ds.T @ q[r0:r1, h]
+    return out, lse, dq, dk, dv
+
+
+def exact(case, seed):
+    if work(case)["flops"] > 2e13:                       # more than about 20 seconds in 64 bits
+        return None
+    s = prepare(case, seed)
+    q, k, v = (t.detach().double() for t in (s.q, s.k, s.v))
+    dout = None if s.dout is None else s.dout.double()
+    if s.kind in ("fwd", "train"):
+        parts = [_attend(q[b], k[b], v[b], None if dout is None else dout[b], s.causal) for b in range(q.size(0))]
+        out, lse, dq, dk, dv = (torch.stack(x) for x in zip(*parts))
+    else:
+        parts = [_attend(*x, s.causal) for x in zip(q.split(s.lens), k.split(s.lens), v.split(s.lens),
+                                                    [None] * len(s.lens) if dout is None else dout.split(s.lens))]
+        out, lse, dq, dk, dv = (torch.cat(x, dim=1 if n == 1 else 0) for n, x in enumerate(zip(*parts)))
+    if s.dout is None:
+        return out, lse
+    if s.kind == "ring" or case.get("api") == "autograd":
+        return out, dq, dk, dv
+    return out, lse, dq, dk, dv
