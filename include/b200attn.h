@@ -78,6 +78,14 @@ typedef struct b2a_fwd_args {
 size_t b2a_fwd_workspace_bytes(int32_t batch, int32_t total_q, int32_t is_varlen);
 
 /*
+ * Scratch with which b2a_fwd is fastest for these arguments on the current device (pointers are not
+ * looked at, except whether cu_seqlens_q is NULL).  Never less than b2a_fwd_workspace_bytes.  It is more
+ * where a fixed-length call has too few query rows to keep every SM busy, e.g. a few tokens against long
+ * K/V: with that much scratch the keys are cut as well and the partial results added up.
+ */
+size_t b2a_fwd_scratch_bytes(const b2a_fwd_args* args);
+
+/*
  * Attention forward: out = softmax(scale * q k^T [+causal]) v, lse = logsumexp.
  * Replaces `forward` (bindings.cpp:240) and `forward_varlen` (bindings.cpp:280)
  * of the reference, including its varlen scheduler-metadata kernel

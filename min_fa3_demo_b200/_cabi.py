@@ -164,6 +164,7 @@ SIGNATURES = {
     "b2a_abi_version": (c_int32, []),
     "b2a_last_error": (c_char_p, []),
     "b2a_fwd_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
+    "b2a_fwd_scratch_bytes": (c_size_t, [POINTER(FwdArgs)]),
     "b2a_fwd": (c_int32, [POINTER(FwdArgs), c_void_p]),
     "b2a_fwd_noalloc": (c_int32, [POINTER(FwdArgs), c_void_p]),
     "b2a_fwd_noalloc_scratch_limit": (c_size_t, []),

@@ -11,7 +11,14 @@
 //   warp  4-7   softmax warpgroup of tile B
 //   warp  8     tcgen05.mma issue
 //   warp  9     TMA loads and work fetch
-//   warp 10-11  idle (they only donate their registers)
+//   warp 10-11  idle (10 stores in the copy roles)
+//
+// What bounds a tile is the chain softmax -> P V -> Q K^T (about 3,300 clk per block and tile against 2 x 1,024 of MMA for
+// the two tiles), so it does not stop between two work items: the first Q K^T of the next item is issued right behind the
+// last P V of the same tile, and the load warp hands out decoded work items through a ring of kFwdSlots, so that no other
+// warp waits for the ticket or for the document table.  With packed rows (fwd_pack_shift) that gives 5 % on 50 documents
+// of about 330 tokens (90.2 -> 85.9 us) and nothing measurable on long ones.  A warpgroup of its own for the epilogue was
+// slower: the softmax warps then have 176 registers instead of 216 and spill (1,750 -> 1,840 us on 4 x 8,192).
 //
 // Tensor memory (512 columns): S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512).
 // P (bf16) overwrites the first 64 columns of its S tile and is consumed by the
@@ -42,6 +49,11 @@ constexpr int kFwdTilesPerCta = 2;   // tiles per work item
 constexpr int kFwdRowsPerWork = kTileM * kFwdTilesPerCta;
 constexpr int kFwdStages = 4;        // K/V ring stages
 constexpr int kFwdThreads = 384;
+constexpr int kFwdSlots = 4;         // decoded work items in flight between the load warp and its consumers
+constexpr int kFwdMmaWarp = 8;
+constexpr int kFwdLoadWarp = 9;
+constexpr int kFwdStoreWarp = 10;    // copy roles only
+constexpr int kFwdMaxSplits = 32;    // pieces of a key split
 constexpr uint32_t kTileBytes = kTileM * kHeadDim * 2;   // 32 KiB bf16 tile
 constexpr uint32_t kHalfTileBytes = kTileBytes / 2;      // one 64-column half
 constexpr float kLog2e = 1.4426950408889634f;
@@ -66,6 +78,16 @@ struct FwdParams {
     int heads_k;
     int causal;
     int num_entries_host;        // BSHD: batch * m_blocks.  varlen: upper bound (unused)
+    int pack_shift;              // log2 of the query heads that share a tile's rows (0: a tile is one head)
+    // Key split (fixed-length calls): behind the first whole_items, an item with more than split_blocks K/V blocks is cut
+    // into up to max_splits pieces that different CTAs compute and fwd_combine_kernel adds up.  Only kFwdSplit launches look at these.
+    int max_splits;
+    int whole_items;
+    int split_blocks;
+    int split_tiles;             // row tiles of an item that hold rows (1 or 2)
+    int split_rows;              // rows of a tile that hold any (at most 128)
+    float2* split_stat;          // [items * max_splits * split_tiles][split_rows] (row maximum, row sum)
+    float4* split_o;             // [items * max_splits * split_tiles][32][split_rows] unnormalised O
     float scale;                 // softmax scale
     float scale_log2;            // scale * log2(e)
     long long lse_head_stride;   // elements between heads
@@ -111,6 +133,7 @@ struct RingDoc {
 struct FwdWork {
     int q_begin;   // first token of the document in the flat Q tensor
     int q_len;
+    int shift;     // a tile is 128 >> shift query rows of 1 << shift heads, row major (heads of one row adjacent)
     int k_begin;
     int k_len;
     int m0;        // first query row (document-local) of the work item
@@ -122,11 +145,17 @@ struct FwdWork {
     int half;      // ring mode: 0 = front half, 1 = back half of the local zigzag shard
     int pair;      // 1: at most 128 rows left -> tiles A / B are heads `head`, `head + 1` of the same rows
                    // (only the even head of each pair carries the work; the odd one's item is empty)
+    int nblk[2];   // K/V blocks of the two tiles (0: no query row, or no visible key)
+    int j0;        // first K/V block (> 0 only for pieces of a key split)
+    int splits;    // pieces of the item (1: not cut)
+    int split;     // which piece this is
+    int item;      // number of the item among those that may be cut
+    int valid;     // 0: no more work
 };
 
-// First row (document-local) and query head of tile x of a work item.
+// First query row (document-local) and query head of tile x of a work item.
 __device__ __forceinline__ int fwd_tile_row0(const FwdWork& wk, int x) {
-    return wk.m0 + (wk.pair ? 0 : x * kTileM);
+    return wk.m0 + (wk.pair ? 0 : x * (kTileM >> wk.shift));
 }
 __device__ __forceinline__ int fwd_tile_head(const FwdWork& wk, int x) {
     return wk.head + (wk.pair ? x : 0);
@@ -134,12 +163,20 @@ __device__ __forceinline__ int fwd_tile_head(const FwdWork& wk, int x) {
 
 // Whether a piece that starts at row m0 of a q_len-row document runs as a pair of heads.
 __device__ __forceinline__ int fwd_pair_mode(const FwdParams& p, int q_len, int m0) {
-    return (q_len - m0 <= kTileM && ((p.heads_q / p.heads_k) & 1) == 0) ? 1 : 0;
+    return (p.pack_shift == 0 && q_len - m0 <= kTileM && ((p.heads_q / p.heads_k) & 1) == 0) ? 1 : 0;
+}
+
+// Work items per entry of the work list.
+__host__ __device__ __forceinline__ int fwd_items_per_entry(const FwdParams& p) {
+    // Packed fixed-length calls list pieces of one item's rows, so an entry is one item per K/V head.  Packed documents
+    // keep the list of 256-row pieces, whose 1 << pack_shift parts are items of their own.
+    return (p.pack_shift > 0 && p.cu_seqlens_q == nullptr) ? p.heads_k : p.heads_q;
 }
 
 struct __align__(1024) FwdShared {
     uint8_t q[kFwdTilesPerCta][kTileBytes];
     uint8_t kv[kFwdStages][kTileBytes];
+    FwdWork work[kFwdSlots];
     uint64_t q_full[kFwdTilesPerCta];
     uint64_t q_empty[kFwdTilesPerCta];
     uint64_t kv_full[kFwdStages];
@@ -147,11 +184,10 @@ struct __align__(1024) FwdShared {
     uint64_t s_full[kFwdTilesPerCta];
     uint64_t p_full[kFwdTilesPerCta];
     uint64_t o_full[kFwdTilesPerCta];
-    uint64_t sched_full[2];
-    uint64_t sched_empty[2];
+    uint64_t sched_full[kFwdSlots];
+    uint64_t sched_empty[kFwdSlots];
     uint64_t comm_full[6];
     uint64_t comm_empty[6];
-    int sched_w[2];
     uint32_t tmem_base;
     uint32_t abort_flag;
 };
@@ -173,14 +209,36 @@ __host__ __device__ __forceinline__ int ring_full_chunks(int causal, int ring_si
     return ring_size;
 }
 
-__device__ __forceinline__ FwdWork fwd_decode_work(const FwdParams& p, int w) {
-    FwdWork wk;
-    int entry = w / p.heads_q;
-    wk.head = w - entry * p.heads_q;
-    wk.head_k = wk.head / (p.heads_q / p.heads_k);
-    wk.n_full = 0;
-    wk.doc = 0;
-    wk.half = 0;
+__device__ __forceinline__ int fwd_num_kv_blocks(const FwdParams& p, const FwdWork& wk, int x);
+
+// Work item w; `valid` = 0 once the tickets have run out.
+template <bool kSplit>
+__device__ __forceinline__ FwdWork fwd_decode_work(const FwdParams& p, int w, int total_work) {
+    FwdWork wk{};
+    if (w >= total_work) return wk;
+    wk.valid = 1;
+    const int per_entry = fwd_items_per_entry(p);
+    wk.splits = 1;
+    const bool cut = kSplit && w >= p.whole_items;
+    if (cut) {
+        // max_splits tickets per item; the pieces that an item does not need come out empty.
+        const int c = w - p.whole_items;
+        wk.item = c / p.max_splits;
+        wk.split = c - wk.item * p.max_splits;
+        w = p.whole_items + wk.item;
+    }
+    int entry = w / per_entry;
+    int part = 0;                        // packed documents: which 256 >> shift rows of the 256-row piece
+    wk.head = w - entry * per_entry;
+    wk.shift = p.pack_shift;
+    if (p.pack_shift > 0) {
+        part = wk.head / p.heads_k;      // 0 for fixed-length calls
+        wk.head_k = wk.head - part * p.heads_k;
+        wk.head = wk.head_k << p.pack_shift;
+        if (p.causal && p.cu_seqlens_q != nullptr) part = (1 << p.pack_shift) - 1 - part;   // longest first
+    } else {
+        wk.head_k = wk.head / (p.heads_q / p.heads_k);
+    }
     if (p.ring_docs != nullptr) {
         const int4 e = p.ring_work[entry];
         const RingDoc& d = p.ring_docs[e.x];
@@ -193,11 +251,9 @@ __device__ __forceinline__ FwdWork fwd_decode_work(const FwdParams& p, int w) {
         wk.m0 = e.z * kFwdRowsPerWork;
         wk.n_full = ring_full_chunks(p.causal, d.ring_size, d.ring_rank, e.y) * (d.half_len / kTileN);
         wk.lse_base = static_cast<long long>(wk.head) * p.lse_head_stride + wk.q_begin;
-        wk.pair = fwd_pair_mode(p, wk.q_len, wk.m0);
-        return wk;
-    }
-    if (p.cu_seqlens_q == nullptr) {
-        int nmb = (p.seqlen_q + kFwdRowsPerWork - 1) / kFwdRowsPerWork;
+    } else if (p.cu_seqlens_q == nullptr) {
+        const int rows = kFwdRowsPerWork >> wk.shift;
+        int nmb = (p.seqlen_q + rows - 1) / rows;
         int b = entry / nmb;
         int mi = entry - b * nmb;
         int mblk = p.causal ? (nmb - 1 - mi) : mi;
@@ -205,7 +261,7 @@ __device__ __forceinline__ FwdWork fwd_decode_work(const FwdParams& p, int w) {
         wk.q_len = p.seqlen_q;
         wk.k_begin = b * p.seqlen_k;
         wk.k_len = p.seqlen_k;
-        wk.m0 = mblk * kFwdRowsPerWork;
+        wk.m0 = mblk * rows;
         wk.lse_base = static_cast<long long>(b) * p.lse_batch_stride +
                       static_cast<long long>(wk.head) * p.lse_head_stride;
     } else {
@@ -215,26 +271,37 @@ __device__ __forceinline__ FwdWork fwd_decode_work(const FwdParams& p, int w) {
         wk.q_len = p.cu_seqlens_q[doc + 1] - wk.q_begin;
         wk.k_begin = p.cu_seqlens_k[doc];
         wk.k_len = p.cu_seqlens_k[doc + 1] - wk.k_begin;
-        wk.m0 = e.y * kFwdRowsPerWork;
+        wk.m0 = e.y * kFwdRowsPerWork + part * (kFwdRowsPerWork >> wk.shift);
         wk.lse_base = static_cast<long long>(wk.head) * p.lse_head_stride + wk.q_begin;
     }
     wk.pair = fwd_pair_mode(p, wk.q_len, wk.m0);
+    wk.nblk[0] = fwd_num_kv_blocks(p, wk, 0);
+    wk.nblk[1] = fwd_num_kv_blocks(p, wk, 1);
+    if (cut) {
+        const int n = max(wk.nblk[0], wk.nblk[1]);
+        wk.splits = min(p.max_splits, max(1, (n + p.split_blocks - 1) / p.split_blocks));
+        if (wk.split >= wk.splits) {
+            wk.m0 = wk.q_len;   // no such piece
+            return wk;
+        }
+        wk.j0 = n * wk.split / wk.splits;
+        const int end = n * (wk.split + 1) / wk.splits;
+        wk.nblk[0] = max(0, min(end, wk.nblk[0]) - wk.j0);
+        wk.nblk[1] = max(0, min(end, wk.nblk[1]) - wk.j0);
+    }
     return wk;
 }
 
 // Number of K/V blocks tile `x` of the work item needs (0 when the tile has no
 // query row, or no visible key).
 __device__ __forceinline__ int fwd_num_kv_blocks(const FwdParams& p, const FwdWork& wk, int x) {
-    if (wk.pair && (wk.head & 1)) {
-        return 0;   // the even head of the pair carries both
-    }
     int row0 = fwd_tile_row0(wk, x);
     if (row0 >= wk.q_len) {
         return 0;
     }
     int limit = wk.k_len;
     if (p.causal) {
-        int row_last = min(row0 + kTileM, wk.q_len) - 1;
+        int row_last = min(row0 + (kTileM >> wk.shift), wk.q_len) - 1;
         limit = min(limit, row_last + 1 + wk.k_len - wk.q_len);
     }
     const int own = limit <= 0 ? 0 : (limit + kTileN - 1) / kTileN;
@@ -314,7 +381,7 @@ __device__ __forceinline__ void ring_copy_role(const FwdParams& p, FwdShared& sh
     const uint32_t slot_base = smem_u32(&sh.q[0][0]);
     const int first = static_cast<int>(blockIdx.x) - p.num_comp;
     const int stride = static_cast<int>(gridDim.x) - p.num_comp;
-    if (warp == 9 && lane == 0) {
+    if (warp == kFwdLoadWarp && lane == 0) {
         uint32_t it = 0;
         bool ok = true;
         for (int t = first; t < p.comm_task_count && ok; t += stride) {
@@ -332,7 +399,7 @@ __device__ __forceinline__ void ring_copy_role(const FwdParams& p, FwdShared& sh
                 }
             }
         }
-    } else if (warp == 10 && lane == 0) {
+    } else if (warp == kFwdStoreWarp && lane == 0) {
         uint32_t it = 0;
         bool ok = true;
         for (int t = first; t < p.comm_task_count && ok; t += stride) {
@@ -378,7 +445,7 @@ __device__ __forceinline__ void prefetch_copy_role(const FwdParams& p, FwdShared
     const long long per_buf = static_cast<long long>((p.prefetch_bytes + kSlotBytes - 1) / kSlotBytes);
     const long long first = static_cast<long long>(blockIdx.x) - p.num_comp;
     const long long stride = static_cast<long long>(gridDim.x) - p.num_comp;
-    if ((warp != 9 && warp != 10) || lane != 0) return;
+    if ((warp != kFwdLoadWarp && warp != kFwdStoreWarp) || lane != 0) return;
     uint32_t it = 0;
     bool ok = true;
     for (long long t = first; t < 2 * per_buf && ok; t += stride, ++it) {
@@ -387,7 +454,7 @@ __device__ __forceinline__ void prefetch_copy_role(const FwdParams& p, FwdShared
         const unsigned long long left = p.prefetch_bytes - off;
         const uint32_t bytes = static_cast<uint32_t>(left < kSlotBytes ? left : kSlotBytes);
         const uint32_t slot = it % 6u;
-        if (warp == 9) {
+        if (warp == kFwdLoadWarp) {
             ok = mbar_wait(wctx, smem_u32(&sh.comm_empty[slot]), ((it / 6u) & 1u) ^ 1u, 27);
             if (!ok) break;
             mbar_arrive_expect_tx(smem_u32(&sh.comm_full[slot]), bytes);
@@ -405,10 +472,14 @@ __device__ __forceinline__ void prefetch_copy_role(const FwdParams& p, FwdShared
             mbar_arrive(smem_u32(&sh.comm_empty[slot]));
         }
     }
-    if (warp == 10) bulk_wait_group<0>();
+    if (warp == kFwdStoreWarp) bulk_wait_group<0>();
 }
 
-template <bool kMerge>
+// What a launch does besides plain attention: merge into a running result, or cut items along their keys.  Kernels of
+// their own, because the softmax warps have no registers to spare for what the plain one does not need.
+enum FwdMode { kFwdPlain = 0, kFwdMerge = 1, kFwdSplit = 2 };
+
+template <int kMode>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
            const __grid_constant__ CUtensorMap map_v, const FwdParams p) {
@@ -431,7 +502,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             mbar_init(smem_u32(&sh.kv_full[i]), 1);
             mbar_init(smem_u32(&sh.kv_empty[i]), 1);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kFwdSlots; ++i) {
             mbar_init(smem_u32(&sh.sched_full[i]), 1);
             mbar_init(smem_u32(&sh.sched_empty[i]), 1 + 2 * 4);  // MMA warp + 8 softmax warps
         }
@@ -443,7 +514,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
         fence_mbar_init();
         fence_proxy_async_smem();
     }
-    if (warp == 8) {
+    if (warp == kFwdMmaWarp) {
         tmem_alloc(smem_u32(&sh.tmem_base), 512);
         tmem_relinquish();
         tc_fence_before_sync();
@@ -453,9 +524,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh.tmem_base);
 
     WaitCtx wctx{smem_u32(&sh.abort_flag), p.status, p.timeout_ns};
-
-    const int total_work =
-        (p.cu_seqlens_q == nullptr ? p.num_entries_host : *p.num_entries_dev) * p.heads_q;
 
     // Copy CTAs (ring mode): pull the other ranks' K/V blocks into the local arena first, then
     // join the attention work queue like every other CTA.
@@ -470,40 +538,44 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
 
     if (warp >= 8) {
         reg_dealloc<72>();
-        if (warp == 9) {
+        if (warp == kFwdLoadWarp) {
             // ------------------------------------------------------------ load warp
             if (lane == 0) {
                 tma_prefetch_desc(&map_q);
                 tma_prefetch_desc(&map_k);
                 tma_prefetch_desc(&map_v);
             }
+            int total_work =
+                (p.cu_seqlens_q == nullptr ? p.num_entries_host : *p.num_entries_dev) * fwd_items_per_entry(p);
+            if (kMode == kFwdSplit) total_work += (total_work - p.whole_items) * (p.max_splits - 1);
             uint32_t kv_it = 0;
             uint32_t q_cnt[2] = {0, 0};
             bool ok = true;
             // Ring mode: true once all copy CTAs are done, i.e. every remote block has landed.
             bool all_landed = p.ring_docs == nullptr || p.comm_task_count == 0;
             const int copy_ctas = static_cast<int>(gridDim.x) - p.num_comp;
+            int ticket = 0;
+            if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);
             for (uint32_t it = 0; ok; ++it) {
-                const uint32_t slot = it & 1u;
-                ok = mbar_wait(wctx, smem_u32(&sh.sched_empty[slot]), ((it >> 1) & 1u) ^ 1u, 1);
+                const uint32_t slot = it % kFwdSlots;
+                ok = mbar_wait(wctx, smem_u32(&sh.sched_empty[slot]), ((it / kFwdSlots) & 1u) ^ 1u, 1);
                 if (!ok) break;
-                int w = 0;
-                if (lane == 0) {
-                    w = atomicAdd(p.sched_counter, 1);
-                    if (w >= total_work) w = -1;
-                    sh.sched_w[slot] = w;
+                FwdWork wk = fwd_decode_work<kMode == kFwdSplit>(p, __shfl_sync(0xFFFFFFFFu, ticket, 0), total_work);
+                while (wk.valid && (wk.m0 >= wk.q_len || (wk.pair && (wk.head & 1)))) {   // no query rows
+                    if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);
+                    wk = fwd_decode_work<kMode == kFwdSplit>(p, __shfl_sync(0xFFFFFFFFu, ticket, 0), total_work);
                 }
-                w = __shfl_sync(0xFFFFFFFFu, w, 0);
                 if (lane == 0) {
+                    sh.work[slot] = wk;
                     mbar_arrive(smem_u32(&sh.sched_full[slot]));
                 }
-                if (w < 0) break;
-                const FwdWork wk = fwd_decode_work(p, w);
-                int nblk[2] = {fwd_num_kv_blocks(p, wk, 0), fwd_num_kv_blocks(p, wk, 1)};
-                const int n_max = max(nblk[0], nblk[1]);
+                if (!wk.valid) break;
+                // The next ticket travels while this item's K/V stream is issued.
+                if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);
+                const int n_max = max(wk.nblk[0], wk.nblk[1]);
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    if (nblk[x] > 0) {
+                    if (wk.nblk[x] > 0) {
                         ok = mbar_wait(wctx, smem_u32(&sh.q_empty[x]), (q_cnt[x] & 1u) ^ 1u, 2);
                         if (!ok) break;
                         ++q_cnt[x];
@@ -525,7 +597,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                                        ((kv_it / kFwdStages) & 1u) ^ 1u, 3);
                         if (!ok) break;
                         ++kv_it;
-                        int row = wk.k_begin + j * kTileN;
+                        int row = wk.k_begin + (wk.j0 + j) * kTileN;
                         if (p.ring_docs != nullptr) {
                             bool remote = false;
                             row = ring_kv_row(p, wk, j, &remote);
@@ -553,7 +625,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                     }
                 }
             }
-        } else if (warp == 8) {
+        } else if (warp == kFwdMmaWarp) {
             // ------------------------------------------------------------ MMA warp
             constexpr uint32_t idesc_qk = make_idesc_bf16(kTileM, kTileN, 0, 0);
             constexpr uint32_t idesc_pv = make_idesc_bf16(kTileM, kHeadDim, 0, 1);
@@ -561,7 +633,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             uint32_t q_cnt[2] = {0, 0};
             uint32_t p_cnt[2] = {0, 0};
             bool ok = true;
-            unsigned long long tile_visits = 0, kv_tile_reads = 0;   // CTA-local totals for p.stats
+            unsigned int tile_visits = 0, kv_tile_reads = 0;   // CTA-local totals for p.stats
             PH_DECL(8)   // 0 other, 1 wait p_full, 2 issue PV, 3 wait K, 4 issue S
             const uint32_t s_tmem[2] = {tmem_base + 0u, tmem_base + 128u};
             const uint32_t o_tmem[2] = {tmem_base + 256u, tmem_base + 384u};
@@ -581,112 +653,137 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 umma_ts_x8_w(o_tmem[x], s_tmem[x], v_lo0 + stage * kStageStep, idesc_pv, accumulate);
             };
 
-            for (uint32_t it = 0; ok; ++it) {
-                const uint32_t slot = it & 1u;
-                ok = mbar_wait(wctx, smem_u32(&sh.sched_full[slot]), (it >> 1) & 1u, 4);
-                if (!ok) break;
-                // Broadcast from lane 0 so that everything derived from the work index (block counts,
-                // ring stages, operand descriptors) is provably warp-uniform for the compiler.
-                const int w = __shfl_sync(0xFFFFFFFFu, *reinterpret_cast<volatile int*>(&sh.sched_w[slot]), 0);
+            auto issue_s = [&](int x, int j, uint32_t stage) {
+                issue_qk(x, stage);
+                tc_commit_w(smem_u32(&sh.s_full[x]));
+                if (j == 0) tc_commit_w(smem_u32(&sh.q_empty[x]));
+            };
+            // First S of tile x in an item with n blocks for it, n_max for the longer tile (whose last block comes first).
+            auto start_tile = [&](int x, int n, int n_max, uint32_t stage) -> bool {
+                if (n == 0) return true;
+                if (!mbar_wait(wctx, smem_u32(&sh.q_full[x]), q_cnt[x] & 1u, 5)) return false;
+                ++q_cnt[x];
+                tc_fence_after_sync();
+                if (n == n_max) issue_s(x, n - 1, stage);
+                return true;
+            };
+            // P V of block j of tile x.
+            auto add_pv = [&](int x, int j, int n, uint32_t stage) -> bool {
+                PH_MARK(0);
+                if (!mbar_wait(wctx, smem_u32(&sh.p_full[x]), p_cnt[x] & 1u, 8)) return false;
+                ++p_cnt[x];
+                tc_fence_after_sync();
+                PH_MARK(1);
+                issue_pv(x, stage, j != n - 1 ? 1u : 0u);
+                if (j == 0) tc_commit_w(smem_u32(&sh.o_full[x]));
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(smem_u32(&sh.sched_empty[slot]));
-                }
-                if (w < 0) break;
-                const FwdWork wk = fwd_decode_work(p, w);
-                int nblk[2] = {fwd_num_kv_blocks(p, wk, 0), fwd_num_kv_blocks(p, wk, 1)};
-                const int n_max = max(nblk[0], nblk[1]);
-                if (n_max == 0) continue;
+                PH_MARK(2);
+#ifdef B2A_PHASES
+                ph_[9] += 1;
+#endif
+                return true;
+            };
+            // Block counts of the next work item; `valid` = 0 when there is none.
+            uint32_t sched_it = 0;
+            auto next_item = [&](int (&n)[2], int& n_max, int& valid) -> bool {
+                const uint32_t slot = sched_it % kFwdSlots;
+                if (!mbar_wait(wctx, smem_u32(&sh.sched_full[slot]), (sched_it / kFwdSlots) & 1u, 4)) return false;
+                ++sched_it;
+                // Broadcast from lane 0 so that everything derived from the counts (ring stages,
+                // operand descriptors) is provably warp-uniform for the compiler.
+                const volatile FwdWork& wk = sh.work[slot];
+                valid = __shfl_sync(0xFFFFFFFFu, wk.valid, 0);
+                n[0] = __shfl_sync(0xFFFFFFFFu, wk.nblk[0], 0);
+                n[1] = __shfl_sync(0xFFFFFFFFu, wk.nblk[1], 0);
+                if (lane == 0) mbar_arrive(smem_u32(&sh.sched_empty[slot]));
+                __syncwarp();
+                n_max = max(n[0], n[1]);
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    if (nblk[x] > 0) {
-                        ok = ok && mbar_wait(wctx, smem_u32(&sh.q_full[x]), q_cnt[x] & 1u, 5);
-                        ++q_cnt[x];
+                    if (n[x] > 0) {
                         tile_visits += 1;
-                        kv_tile_reads += static_cast<unsigned long long>(nblk[x]);
+                        kv_tile_reads += static_cast<unsigned int>(n[x]);
                     }
                 }
-                if (!ok) break;
-                // Prologue: S(j0) for every tile that owns block j0.
-                {
-                    const int j0 = n_max - 1;
+                return true;
+            };
+            int nblk[2] = {0, 0}, n_max = 0, valid = 1;
+            bool started = false;    // the item's first S has been issued behind the previous item's last P V
+            while (ok) {
+                if (!started) {
+                    while (ok && valid && n_max == 0) ok = next_item(nblk, n_max, valid);
+                    if (!ok || !valid) break;
                     const uint32_t stage = kv_it % kFwdStages;
                     ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage]), (kv_it / kFwdStages) & 1u, 6);
                     if (!ok) break;
                     ++kv_it;
-                    tc_fence_after_sync();
-                    {
-#pragma unroll
-                        for (int x = 0; x < 2; ++x) {
-                            if (j0 < nblk[x]) {
-                                issue_qk(x, stage);
-                                tc_commit_w(smem_u32(&sh.s_full[x]));
-                                if (j0 == 0) tc_commit_w(smem_u32(&sh.q_empty[x]));
-                            }
-                        }
-                        tc_commit_w(smem_u32(&sh.kv_empty[stage]));
-                    }
-                    __syncwarp();
+                    ok = start_tile(0, nblk[0], n_max, stage) && start_tile(1, nblk[1], n_max, stage);
+                    tc_commit_w(smem_u32(&sh.kv_empty[stage]));
                 }
-                for (int j = n_max - 1; j >= 0 && ok; --j) {
+                for (int j = n_max - 1; j > 0 && ok; --j) {
                     const uint32_t stage_v = kv_it % kFwdStages;
-                    ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_v]),
-                                   (kv_it / kFwdStages) & 1u, 7);
+                    ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_v]), (kv_it / kFwdStages) & 1u, 7);
                     if (!ok) break;
                     ++kv_it;
-                    uint32_t stage_k = 0;
-                    if (j > 0) {
-                        stage_k = kv_it % kFwdStages;
-                    }
+                    const uint32_t stage_k = kv_it % kFwdStages;
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
                         if (j < nblk[x]) {
-                            PH_MARK(0);
-                            ok = mbar_wait(wctx, smem_u32(&sh.p_full[x]), p_cnt[x] & 1u, 8);
+                            ok = add_pv(x, j, nblk[x], stage_v);
                             if (!ok) break;
-                            ++p_cnt[x];
+                        }
+                        if (x == 1) tc_commit_w(smem_u32(&sh.kv_empty[stage_v]));
+                        if (x == 0) {
+                            ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_k]), (kv_it / kFwdStages) & 1u, 9);
+                            if (!ok) break;
                             tc_fence_after_sync();
-                            PH_MARK(1);
-                            {
-                                issue_pv(x, stage_v, j != nblk[x] - 1 ? 1u : 0u);
-                                if (j == 0) tc_commit_w(smem_u32(&sh.o_full[x]));
-                            }
-                            __syncwarp();
-                            PH_MARK(2);
-#ifdef B2A_PHASES
-                            ph_[9] += 1;
-#endif
                         }
-                        if (x == 1) {
-                            tc_commit_w(smem_u32(&sh.kv_empty[stage_v]));
-                        }
-                        if (j > 0) {
-                            if (x == 0) {
-                                ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_k]),
-                                               (kv_it / kFwdStages) & 1u, 9);
-                                if (!ok) break;
-                                tc_fence_after_sync();
-                            }
-                            PH_MARK(3);
-                            if (j - 1 < nblk[x]) {
-                                issue_qk(x, stage_k);
-                                tc_commit_w(smem_u32(&sh.s_full[x]));
-                                if (j - 1 == 0) tc_commit_w(smem_u32(&sh.q_empty[x]));
-                            }
-                            if (x == 1) {
-                                tc_commit_w(smem_u32(&sh.kv_empty[stage_k]));
-                            }
-                            __syncwarp();
-                            PH_MARK(4);
-                        }
+                        PH_MARK(3);
+                        if (j - 1 < nblk[x]) issue_s(x, j - 1, stage_k);
+                        if (x == 1) tc_commit_w(smem_u32(&sh.kv_empty[stage_k]));
+                        __syncwarp();
+                        PH_MARK(4);
                     }
-                    if (j > 0) ++kv_it;
+                    ++kv_it;
                 }
+                if (!ok) break;
+                // Last block, with the next item's first S behind it.  Only the one item behind this: looking past items
+                // without keys here could mean waiting for softmax warps that wait for tile B below.
+                int nblk_next[2] = {0, 0}, n_max_next = 0;
+                const uint32_t stage_v = kv_it % kFwdStages;
+                ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_v]), (kv_it / kFwdStages) & 1u, 7);
+                if (!ok) break;
+                ++kv_it;
+                const uint32_t stage_k = kv_it % kFwdStages;
+                if (nblk[0] > 0) ok = add_pv(0, 0, nblk[0], stage_v);
+                ok = ok && next_item(nblk_next, n_max_next, valid);
+                if (!ok) break;
+                if (n_max_next > 0) {
+                    ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_k]), (kv_it / kFwdStages) & 1u, 9) &&
+                         start_tile(0, nblk_next[0], n_max_next, stage_k);
+                    if (!ok) break;
+                    __syncwarp();
+                }
+                if (nblk[1] > 0) ok = add_pv(1, 0, nblk[1], stage_v);
+                if (!ok) break;
+                tc_commit_w(smem_u32(&sh.kv_empty[stage_v]));
+                if (n_max_next > 0) {
+                    ok = start_tile(1, nblk_next[1], n_max_next, stage_k);
+                    if (!ok) break;
+                    tc_commit_w(smem_u32(&sh.kv_empty[stage_k]));
+                    __syncwarp();
+                    ++kv_it;
+                }
+                nblk[0] = nblk_next[0];
+                nblk[1] = nblk_next[1];
+                n_max = n_max_next;
+                started = n_max > 0;
+                if (!valid) break;
             }
             // Each CTA submits its two totals once (reference: include/min_fa3_kernel.h:618-625).
             if (p.stats != nullptr && lane == 0 && tile_visits != 0) {
-                atomicAdd(p.stats, tile_visits);
-                atomicAdd(p.stats + 1, kv_tile_reads);
+                atomicAdd(p.stats, static_cast<unsigned long long>(tile_visits));
+                atomicAdd(p.stats + 1, static_cast<unsigned long long>(kv_tile_reads));
             }
             PH_PRINT("fwd mma", 5);
         }
@@ -705,25 +802,33 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
         PH_DECL(8)   // 0 other, 1 wait s_full, 2 tmem load, 3 max/rescale, 4 exp + store, 5 st wait + arrive
 
         for (uint32_t it = 0; ok; ++it) {
-            const uint32_t slot = it & 1u;
-            ok = mbar_wait(wctx, smem_u32(&sh.sched_full[slot]), (it >> 1) & 1u, 10);
+            const uint32_t slot = it % kFwdSlots;
+            ok = mbar_wait(wctx, smem_u32(&sh.sched_full[slot]), (it / kFwdSlots) & 1u, 10);
             if (!ok) break;
-            const int w = *reinterpret_cast<volatile int*>(&sh.sched_w[slot]);
+            const FwdWork wk = sh.work[slot];
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(smem_u32(&sh.sched_empty[slot]));
             }
-            if (w < 0) break;
-            const FwdWork wk = fwd_decode_work(p, w);
+            if (!wk.valid) break;
             const int tile_row0 = fwd_tile_row0(wk, x);
-            if (tile_row0 >= wk.q_len || (wk.pair && (wk.head & 1))) continue;
-            const int nblk = fwd_num_kv_blocks(p, wk, x);
-            const int row = tile_row0 + r;
-            const bool row_valid = row < wk.q_len;
-            const long long tok = static_cast<long long>(wk.q_begin) + row;
-            const int tile_head = fwd_tile_head(wk, x);
-            __nv_bfloat16* o_row = p.o + (tok * p.heads_q + tile_head) * kHeadDim;
-            float* lse_ptr = p.lse + wk.lse_base + static_cast<long long>(tile_head - wk.head) * p.lse_head_stride + row;
+            const int tile_rows = (wk.q_len - tile_row0) << wk.shift;   // rows of the tile that exist (may exceed 128)
+            if (tile_rows <= 0) continue;
+            const int nblk = x == 0 ? wk.nblk[0] : wk.nblk[1];
+            if ((r & ~31) >= tile_rows) {
+                // None of the warp's rows exists: it only keeps step with the barriers.  Its P and O are never looked at.
+                for (int j = nblk - 1; j >= 0 && ok; --j) {
+                    ok = mbar_wait(wctx, smem_u32(&sh.s_full[x]), s_cnt & 1u, 11);
+                    if (!ok) break;
+                    ++s_cnt;
+                    mbar_arrive(smem_u32(&sh.p_full[x]));
+                }
+                if (nblk > 0) ++o_cnt;
+                continue;
+            }
+            const int row = tile_row0 + (r >> wk.shift);
+            const bool row_valid = r < tile_rows;
+            const int tile_head = fwd_tile_head(wk, x) + (r & ((1 << wk.shift) - 1));
 
             // Key columns [0, col_limit) are visible to this row.
             int col_limit = wk.k_len;
@@ -735,6 +840,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             if (p.causal) {
                 tile_min_limit = min(tile_min_limit, tile_row0 + 1 + wk.k_len - wk.q_len);
             }
+            const int n_full = wk.n_full - wk.j0;   // blocks are counted from the piece's first one
 
             float m_used = -INFINITY;   // running reference max (raw score units)
             float l = 0.f;              // running row sum relative to m_used
@@ -758,8 +864,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 tmem_wait_ld();
                 PH_MARK(2);
 
-                const int n0 = (j - wk.n_full) * kTileN;   // own-chunk column of the block
-                if (j >= wk.n_full && n0 + kTileN > tile_min_limit) {
+                const int n0 = (j - n_full) * kTileN;   // own-chunk column of the block
+                if (j >= n_full && n0 + kTileN > tile_min_limit) {
                     const int lim = col_limit - n0;
 #pragma unroll
                     for (int i = 0; i < kTileN; ++i) {
@@ -859,7 +965,34 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 }
             }
 
-            if constexpr (kMerge) {
+            const long long tok = static_cast<long long>(wk.q_begin) + row;
+            __nv_bfloat16* o_row = p.o + (tok * p.heads_q + tile_head) * kHeadDim;
+            float* lse_ptr = p.lse + wk.lse_base + static_cast<long long>(tile_head - wk.head) * p.lse_head_stride + row;
+            if (kMode == kFwdSplit && wk.splits > 1) {
+                // Key split: every piece stores its unnormalised O with the row statistics; fwd_combine_kernel adds the
+                // pieces up.
+                const int rows = p.split_rows;
+                const long long at = (static_cast<long long>(wk.item * p.max_splits + wk.split) * p.split_tiles + x) * rows + r;
+                if (row_valid) p.split_stat[at] = make_float2(m_used, l);
+                float4* dst = p.split_o + (at - r) * 32 + r;
+#pragma unroll
+                for (int c = 0; c < 4 && nblk > 0; ++c) {
+                    uint32_t t[32];
+                    tmem_ld_x32(o_tmem + c * 32, t);
+                    tmem_wait_ld();
+                    if (row_valid) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            dst[(c * 8 + i) * rows] = make_float4(__uint_as_float(t[4 * i]), __uint_as_float(t[4 * i + 1]),
+                                                                  __uint_as_float(t[4 * i + 2]), __uint_as_float(t[4 * i + 3]));
+                        }
+                    }
+                }
+                tc_fence_before_sync();
+                continue;
+            }
+
+            if constexpr (kMode == kFwdMerge) {
                 // Merge this call's (O_b, L_b) into the running (O_p, L_p):
                 //   L = logaddexp(L_p, L_b);  O = O_p * e^(L_p - L) + O_b * e^(L_b - L)
                 float lse_prev = row_valid ? *lse_ptr : -INFINITY;
@@ -941,7 +1074,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     // Common exit: every role arrives here (normally or after an abort).
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 8) {
+    if (warp == kFwdMmaWarp) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }

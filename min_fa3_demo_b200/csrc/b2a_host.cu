@@ -104,7 +104,7 @@ EncodeTiledFn get_encode_fn() {
 }  // namespace
 
 int make_token_map(CUtensorMap* map, const void* base, uint64_t tokens, uint64_t heads,
-                   uint32_t box_rows) {
+                   uint32_t box_rows, uint32_t box_heads) {
     EncodeTiledFn encode = get_encode_fn();
     if (encode == nullptr) {
         return fail(B2A_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
@@ -117,7 +117,7 @@ int make_token_map(CUtensorMap* map, const void* base, uint64_t tokens, uint64_t
     }
     cuuint64_t dims[3] = {128, heads, tokens};
     cuuint64_t strides[2] = {256, heads * 256};
-    cuuint32_t box[3] = {64, 1, box_rows};
+    cuuint32_t box[3] = {64, box_heads, box_rows};
     cuuint32_t elem_strides[3] = {1, 1, 1};
     CUresult res = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
                           strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -44,9 +44,9 @@ struct DeviceInfo {
 int current_device_info(DeviceInfo* info);
 
 // 3-D tiled tensor map over a flat bf16 [tokens, heads, 128] tensor with a
-// (64 columns, 1 head, box_rows tokens) box and 128-byte swizzle.
+// (64 columns, box_heads heads, box_rows tokens) box and 128-byte swizzle.
 int make_token_map(CUtensorMap* map, const void* base, uint64_t tokens, uint64_t heads,
-                   uint32_t box_rows);
+                   uint32_t box_rows, uint32_t box_heads = 1);
 
 // Header words at the start of every workspace.
 struct WorkspaceHeader {
@@ -81,8 +81,8 @@ int noalloc_scratch_ptr(void** out);
 // Returns fn's code the first time and B2A_OK afterwards.
 int once_per_device(int device, int slot, int (*fn)());
 
-// Raises the dynamic shared-memory limit of the forward kernel once per device (b2a_fwd.cu).
-int configure_fwd_kernel(const DeviceInfo& dev, bool merge);
+// Raises the dynamic shared-memory limit of the forward kernel in a FwdMode once per device (b2a_fwd.cu).
+int configure_fwd_kernel(const DeviceInfo& dev, int mode);
 
 // Planner launch (b2a_plan.cu).  kind 0: forward items (256 query rows of a
 // document, cost = visible key blocks).  kind 1: backward items (128 key rows

@@ -173,10 +173,10 @@ int b2a_ring_fwd(const b2a_ring_fwd_args* a, void* cuda_stream) {
     int grid = a->num_comp_sm + comm;
     p.num_comp = a->num_comp_sm;
 
-    rc = configure_fwd_kernel(dev, false);
+    rc = configure_fwd_kernel(dev, kFwdPlain);
     if (rc != B2A_OK) return rc;
     profile_mark(B2A_KERNEL_FWD, false, stream);
-    fwd_kernel<false><<<grid, kFwdThreads, kRingFwdSmemBytes, stream>>>(map_q, map_k, map_v, p);
+    fwd_kernel<kFwdPlain><<<grid, kFwdThreads, kRingFwdSmemBytes, stream>>>(map_q, map_k, map_v, p);
     profile_mark(B2A_KERNEL_FWD, true, stream);
     B2A_CUDA_OK(cudaGetLastError());
     return B2A_OK;

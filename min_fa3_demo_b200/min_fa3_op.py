@@ -186,8 +186,6 @@ def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads
     lib = _cabi.load()
     total_q = q.numel() // (heads_q * 128)
     total_k = k.numel() // (heads_k * 128)
-    nbytes = lib.b2a_fwd_workspace_bytes(batch, total_q, 0 if cu_q is None else 1)
-    ws = _workspace(nbytes, q.device)
     args = _cabi.FwdArgs()
     args.q, args.k, args.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
     args.out, args.lse = out.data_ptr(), lse.data_ptr()
@@ -199,7 +197,6 @@ def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads
     args.merge_running = int(bool(merge_running))
     args.grid_blocks = int(grid_blocks or 0)
     args.softmax_scale = 0.0
-    args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
     if prefetch is not None:
         src_k, src_v, dst_k, dst_v, blocks = prefetch
         args.prefetch_src_k, args.prefetch_src_v = src_k, src_v
@@ -207,6 +204,9 @@ def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads
         args.prefetch_bytes = dst_k.numel() * dst_k.element_size()
         args.prefetch_blocks = int(blocks)
     with torch.cuda.device(q.device):
+        nbytes = lib.b2a_fwd_scratch_bytes(ctypes.byref(args))
+        ws = _workspace(nbytes, q.device)
+        args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
         _cabi.check(lib.b2a_fwd(ctypes.byref(args), _stream_ptr(q.device)))
     return ws
 
@@ -216,9 +216,6 @@ def _call_bwd(dout, q, k, v, out, lse, dq, dk, dv, *, cu_q, cu_k, batch, seqlen_
     lib = _cabi.load()
     total_q = q.numel() // (heads_q * 128)
     total_k = k.numel() // (heads_k * 128)
-    nbytes = lib.b2a_bwd_workspace_bytes(batch, total_q, total_k, heads_q, heads_k,
-                                         0 if cu_q is None else 1)
-    ws = _workspace(nbytes, q.device)
     args = _cabi.BwdArgs()
     args.dout, args.q, args.k, args.v = dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
     args.out, args.lse = out.data_ptr(), lse.data_ptr()
@@ -231,8 +228,11 @@ def _call_bwd(dout, q, k, v, out, lse, dq, dk, dv, *, cu_q, cu_k, batch, seqlen_
     args.deterministic = int(bool(deterministic))
     args.grid_blocks = 0
     args.softmax_scale = 0.0
-    args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
     with torch.cuda.device(q.device):
+        nbytes = lib.b2a_bwd_workspace_bytes(batch, total_q, total_k, heads_q, heads_k,
+                                             0 if cu_q is None else 1)
+        ws = _workspace(nbytes, q.device)
+        args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
         _cabi.check(lib.b2a_bwd(ctypes.byref(args), _stream_ptr(q.device)))
     return ws
 

@@ -3,10 +3,14 @@ oracle and the reference's golden fixtures.  Acceptance: O within 2x the max-abs
 bf16 PyTorch attention against the fp32 oracle, LSE within 1e-3 absolute."""
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 
 import min_fa3_op
+from min_fa3_demo_b200 import _cabi
+from min_fa3_demo_b200 import min_fa3_op as min_fa3_op_impl
 from conftest import from_bf16_bits, load_golden
 from gpu_util import (assert_lse, assert_within, bound, make_bshd, make_varlen, varlen_bf16_errors)
 from oracle import attention_oracle as orc
@@ -51,6 +55,47 @@ def test_bshd_forward_rectangular_causal(sq, sk):
     assert_lse(lse, ref_lse)
     if sq > sk:
         assert torch.all(out[0, : sq - sk] == 0)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("b,sq,sk,qh,kvh", [
+    (1, 1, 1024, 8, 1),       # one row of 8 heads: one tile, 8 of its rows used, keys cut into many pieces
+    (2, 1, 4001, 8, 2),       # ... with a ragged last key block
+    (1, 31, 2049, 16, 4),     # 124 packed rows
+    (1, 33, 3000, 16, 4),     # 132: four rows in the second tile
+    (1, 300, 4096, 4, 4),     # nothing to pack; the second item has 44 rows
+    (1, 200, 5000, 32, 1),    # 32 heads a row: four rows a tile
+    (1, 1030, 2048, 8, 2),    # causal: items of different lengths, cut into different numbers of pieces
+    (1, 100, 3000, 12, 2),    # groups of 6 are not packed and not cut: two heads an item
+    (1, 90, 1100, 6, 2),      # groups of 3
+    (1, 700, 1024, 256, 1),   # more heads than a tile has rows
+    (1, 9000, 70, 40, 40),    # causal: CTAs draw many items in a row that see no key
+    (1, 4500, 70, 24, 4),     # ... of two heads each
+])
+def test_bshd_forward_packed_rows_and_key_pieces(b, sq, sk, qh, kvh, causal):
+    q, k, v, _ = make_bshd(31 + sq, b, sq, qh, kvh, sk=sk)
+    out, lse = run_bshd(q, k, v, causal)
+    min_fa3_op_impl.check_last_status("forward")
+    ref_out, ref_lse = orc.bshd_forward(q, k, v, causal)
+    e = orc.bf16_attention_error(q, k, v, causal)["o"]
+    assert_within("O", out, ref_out, e)
+    assert_lse(lse, ref_lse)
+    # The plain workspace is enough for the same call, without cutting the keys.
+    lib = _cabi.load()
+    a = _cabi.FwdArgs()
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    out2, lse2 = torch.empty_like(qd), torch.empty_like(lse)
+    a.q, a.k, a.v, a.out, a.lse = (t.data_ptr() for t in (qd, kd, vd, out2, lse2))
+    a.batch, a.seqlen_q, a.seqlen_k, a.total_q, a.total_k = b, sq, sk, b * sq, b * sk
+    a.heads_q, a.heads_k, a.head_dim, a.is_causal = qh, kvh, 128, int(causal)
+    plain = lib.b2a_fwd_workspace_bytes(b, b * sq, 0)
+    assert lib.b2a_fwd_scratch_bytes(ctypes.byref(a)) >= plain
+    ws = torch.empty(plain, dtype=torch.uint8, device="cuda")
+    a.workspace, a.workspace_bytes = ws.data_ptr(), plain
+    _cabi.check(lib.b2a_fwd(ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    assert_within("O (plain workspace)", out2, ref_out, e)
+    assert_lse(lse2, ref_lse)
 
 
 @pytest.mark.parametrize("tag,causal", [("full", False), ("causal", True)])
