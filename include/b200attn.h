@@ -163,6 +163,13 @@ size_t b2a_bwd_workspace_bytes(int32_t batch, int32_t total_q, int32_t total_k, 
                                int32_t heads_k, int32_t is_varlen);
 
 /*
+ * Scratch with which b2a_bwd is fastest for these arguments on the current device (see b2a_fwd_scratch_bytes).
+ * Never less than b2a_bwd_workspace_bytes; more where a fixed-length call has too few key blocks to keep
+ * every SM busy: the query tiles are then cut as well and the partial dK / dV added up.
+ */
+size_t b2a_bwd_scratch_bytes(const b2a_bwd_args* args);
+
+/*
  * Attention backward: dq, dk, dv from dout and the forward's q, k, v, out, lse.
  * Replaces `backward` (csrc/backward/min_fa3_bwd_bindings.cu:156) and
  * `backward_varlen` (csrc/backward/min_fa3_bwd_bindings.cu:255): the dO*O

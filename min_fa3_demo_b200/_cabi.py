@@ -168,6 +168,7 @@ SIGNATURES = {
     "b2a_fwd": (c_int32, [POINTER(FwdArgs), c_void_p]),
     "b2a_fwd_noalloc": (c_int32, [POINTER(FwdArgs), c_void_p]),
     "b2a_fwd_noalloc_scratch_limit": (c_size_t, []),
+    "b2a_bwd_scratch_bytes": (c_size_t, [POINTER(BwdArgs)]),
     "b2a_bwd_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32, c_int32, c_int32, c_int32]),
     "b2a_bwd": (c_int32, [POINTER(BwdArgs), c_void_p]),
     "b2a_ipc_export": (c_int32, [c_void_p, c_void_p, POINTER(ctypes.c_uint64)]),

@@ -3,6 +3,7 @@
 #include "b2a_host.cuh"
 #include "b2a_ring_host.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -63,18 +64,125 @@ BwdLayout bwd_layout(int batch, int seqlen_q, int total_q, int total_k, int head
     return l;
 }
 
+template <bool kSplit>
 int set_bwd_smem_attribute() {
-    B2A_CUDA_OK(cudaFuncSetAttribute(bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    B2A_CUDA_OK(cudaFuncSetAttribute(bwd_kernel<kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kBwdSmemBytes)));
     return B2A_OK;
 }
 
-int configure_bwd_kernel(const DeviceInfo& dev) {
+int configure_bwd_kernel(const DeviceInfo& dev, bool split) {
     if (static_cast<size_t>(dev.max_smem_optin) < kBwdSmemBytes) {
         return fail(B2A_ERR_UNSUPPORTED_DEVICE, "device offers %d bytes of shared memory, need %zu",
                     dev.max_smem_optin, kBwdSmemBytes);
     }
-    return once_per_device(dev.device, 2, set_bwd_smem_attribute);
+    return split ? once_per_device(dev.device, 3, set_bwd_smem_attribute<true>)
+                 : once_per_device(dev.device, 2, set_bwd_smem_attribute<false>);
+}
+
+// How a fixed-length call is cut along the steps of its items.  max_splits = 1: not at all.  As in the forward, the
+// caller's own CTA count does not enter.
+struct BwdSplit {
+    int max_splits = 1, whole_items = 0, steps = 0;
+    long long items = 0;         // behind whole_items
+    size_t total() const { return max_splits > 1 ? items * max_splits * 2 * kTileN * kHeadDim * sizeof(float) : 0; }
+};
+
+// An item is one key block of one K/V head with all query tiles of the group that see it.  Where there are few items, or
+// they fill the CTAs unevenly, the query tiles are cut as well.  The cost of k pieces per item, in steps of a CTA (about
+// 2.1 us each), is the number of rounds times the piece, plus two steps a round for starting and storing a piece, two for
+// the launch that adds up, and the time that writing and reading 128 KiB a piece takes (about 4 TB/s).  As in the
+// forward, items of one length run in rounds and only the last, incomplete one is cut; items that differ (causal) are
+// packed by the dynamic hand-out, which the mean load plus half a piece bounds.  A cut has to promise a tenth: the kernel
+// that can cut spills a little, and its steps take 1 to 2 % longer.  Measured (us, whole backward, not cut / cut): 2 x
+// 1,024 causal, 16 over 4 heads: 100 / 80; 1 x 4,096 causal, 8 over 2: 376 / 195; 1 x 2,048, 8 over 1: 305 / 85; 2 x
+// 3,001, 32 heads, the last of eleven rounds cut, which this leaves alone: 820 / 830.
+BwdSplit plan_bwd_split(const b2a_bwd_args& a, int ctas) {
+    BwdSplit s;
+    if (a.cu_seqlens_q != nullptr) return s;
+    const long long nnb = (a.seqlen_k + kTileN - 1) / kTileN;
+    const long long items = nnb * a.batch * a.heads_k;
+    const int group = a.heads_q / a.heads_k;
+    const int tiles = (a.seqlen_q + kTileM - 1) / kTileM;
+    const long long n = static_cast<long long>(tiles) * group;   // steps of the longest item
+    if (n < 4 || items >= 16ll * ctas) return s;
+    double mean = 0;
+    for (long long i = 0; i < nnb; ++i) {
+        const long long first_row = std::max<long long>(0, i * kTileN + a.seqlen_q - a.seqlen_k);
+        mean += static_cast<double>(tiles - (a.is_causal ? std::min<long long>(tiles, first_row / kTileM) : 0));
+    }
+    mean *= static_cast<double>(group) / static_cast<double>(nnb);
+    const bool even = mean > 0.8 * n;
+    const long long whole = even ? items / ctas * ctas : 0;
+    const double cut = static_cast<double>(items - whole);
+    if (cut == 0) return s;
+    auto cost = [&](int k) {
+        const double piece = (n + k - 1) / k, extra = k > 1 ? 2.0 : 0.0, add = k > 1 ? 2.0 + cut * k / 32.0 : 0.0;
+        const double load = cut * k / ctas;
+        if (even) return static_cast<double>(whole / ctas) * n + std::ceil(load) * (piece + extra) + add;
+        return std::max(piece, cut * mean / ctas) + 0.5 * piece + extra * load + add;
+    };
+    int best = 1;
+    for (int k = 2; k <= kBwdMaxSplits && n / k >= 2; ++k) {
+        if (cost(k) < cost(best)) best = k;
+    }
+    if (best == 1 || cost(best) > 0.9 * cost(1)) return s;
+    s.max_splits = best;
+    s.whole_items = static_cast<int>(whole);
+    s.steps = static_cast<int>((n + best - 1) / best);
+    s.items = items - whole;
+    return s.total() > (128u << 20) ? BwdSplit{} : s;   // the caller's thread keeps the scratch of its latest call
+}
+
+// Adds up the pieces of cut items, in the order of their steps, and writes dV and dK * scale.  One CTA per 32 key rows of
+// one of the two; bound by reading the pieces from L2, see fwd_combine_kernel.
+constexpr int kBwdCombineRows = 32;
+
+__global__ void __launch_bounds__(256)
+bwd_combine_kernel(const BwdParams p) {
+    constexpr int kPitch = kHeadDim + 4;    // bf16; keeps the 8-byte column stores of 16 rows on distinct banks
+    __shared__ __align__(8) __nv_bfloat16 out[kBwdCombineRows * kPitch];
+    constexpr int kStrips = kTileN / kBwdCombineRows;
+    const int first = static_cast<int>(blockIdx.x % kStrips) * kBwdCombineRows;
+    const int which = blockIdx.x / kStrips % 2;      // 0: dV, 1: dK
+    const int item = blockIdx.x / (2 * kStrips);
+    const BwdWork wk = bwd_decode_work<true>(p, p.whole_items + item * p.max_splits);
+    const int rows = min(kBwdCombineRows, wk.k_len - wk.n0 - first);
+    if (wk.splits <= 1 || rows <= 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float mul = which == 0 ? 1.f : p.scale;
+    {
+        // Lane = row, four of the 32 column quads a warp.  (Rows beyond k_len were stored as well: zeros.)
+        const float4* src = p.split_part + (static_cast<long long>(item) * p.max_splits * 2 + which) * (32 * kTileN) + first + lane;
+        float4 acc[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+        for (int i = 0; i < wk.splits; ++i) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = __ldcs(src + (static_cast<long long>(i) * 2 * 32 + warp * 4 + u) * kTileN);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                acc[u].x += v[u].x;
+                acc[u].y += v[u].y;
+                acc[u].z += v[u].z;
+                acc[u].w += v[u].w;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            *reinterpret_cast<uint2*>(&out[lane * kPitch + (warp * 4 + u) * 4]) =
+                make_uint2(pack_bf16x2(acc[u].x * mul, acc[u].y * mul), pack_bf16x2(acc[u].z * mul, acc[u].w * mul));
+        }
+    }
+    __syncthreads();
+    // A warp writes one whole 256-byte row per instruction.
+    __nv_bfloat16* dst = which == 0 ? p.dv : p.dk;
+    for (int rr = warp; rr < rows; rr += 8) {
+        const long long to = (static_cast<long long>(wk.k_begin) + wk.n0 + first + rr) * p.heads_k + wk.head_k;
+        *reinterpret_cast<uint2*>(dst + to * kHeadDim + lane * 4) = *reinterpret_cast<const uint2*>(&out[rr * kPitch + lane * 4]);
+    }
 }
 
 }  // namespace
@@ -89,6 +197,19 @@ size_t b2a_bwd_workspace_bytes(int32_t batch, int32_t total_q, int32_t total_k, 
     // For BSHD the padded length is derived from seqlen_q = total_q / batch.
     const int seqlen_q = batch > 0 ? total_q / batch : total_q;
     return b2a::bwd_layout(batch, seqlen_q, total_q, total_k, heads_q, is_varlen != 0).total;
+}
+
+size_t b2a_bwd_scratch_bytes(const b2a_bwd_args* a) {
+    using namespace b2a;
+    if (a == nullptr) return 0;
+    const size_t need = b2a_bwd_workspace_bytes(a->batch, a->total_q, a->total_k, a->heads_q, a->heads_k,
+                                                a->cu_seqlens_q != nullptr ? 1 : 0);
+    DeviceInfo dev{};
+    if (a->batch < 1 || a->heads_q < 1 || a->heads_k < 1 || a->heads_q % a->heads_k != 0 || a->seqlen_q < 1 ||
+        a->seqlen_k < 1 || current_device_info(&dev) != B2A_OK) {
+        return need;   // b2a_bwd reports what is wrong
+    }
+    return need + plan_bwd_split(*a, dev.sm_count).total();
 }
 
 int b2a_bwd(const b2a_bwd_args* a, void* cuda_stream) {
@@ -123,7 +244,9 @@ int b2a_bwd(const b2a_bwd_args* a, void* cuda_stream) {
     DeviceInfo dev{};
     int rc = current_device_info(&dev);
     if (rc != B2A_OK) return rc;
-    rc = configure_bwd_kernel(dev);
+    BwdSplit split = plan_bwd_split(*a, dev.sm_count);
+    if (a->workspace_bytes < lay.total + split.total()) split = BwdSplit{};   // b2a_bwd_workspace_bytes is enough to run
+    rc = configure_bwd_kernel(dev, split.max_splits > 1);
     if (rc != B2A_OK) return rc;
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
 
@@ -222,12 +345,22 @@ int b2a_bwd(const b2a_bwd_args* a, void* cuda_stream) {
         const int nnb = (a->seqlen_k + kTileN - 1) / kTileN;
         p.num_entries_host = a->batch * nnb;
         work_items = static_cast<long long>(p.num_entries_host) * a->heads_k;
+        work_items += (work_items - split.whole_items) * (split.max_splits - 1);
     }
+    p.max_splits = split.max_splits;
+    p.whole_items = split.whole_items;
+    p.split_steps = split.steps;
+    p.split_part = reinterpret_cast<float4*>(ws + lay.total);
     int grid = a->grid_blocks > 0 ? a->grid_blocks : dev.sm_count;
     if (work_items < grid) grid = static_cast<int>(work_items);
     if (grid < 1) grid = 1;
     profile_mark(B2A_KERNEL_BWD, false, stream);
-    bwd_kernel<<<grid, kBwdThreads, kBwdSmemBytes, stream>>>(map_q, map_k, map_v, map_do, p);
+    if (split.max_splits > 1) {
+        bwd_kernel<true><<<grid, kBwdThreads, kBwdSmemBytes, stream>>>(map_q, map_k, map_v, map_do, p);
+        bwd_combine_kernel<<<static_cast<unsigned int>(split.items * 2 * (kTileN / kBwdCombineRows)), 256, 0, stream>>>(p);
+    } else {
+        bwd_kernel<false><<<grid, kBwdThreads, kBwdSmemBytes, stream>>>(map_q, map_k, map_v, map_do, p);
+    }
     profile_mark(B2A_KERNEL_BWD, true, stream);
     B2A_CUDA_OK(cudaGetLastError());
 
@@ -459,14 +592,14 @@ int b2a_ring_bwd(const b2a_ring_bwd_args* a, void* cuda_stream) {
         p.done_ctas = &hdr->reserved;
         p.world = world;
 
-        rc = configure_bwd_kernel(dev);
+        rc = configure_bwd_kernel(dev, false);
         if (rc != B2A_OK) return rc;
         // Without copies the extra CTAs are attention CTAs like the others (sharded documents
         // only: a launch that never had copy tasks keeps its grid).
         const int comm = plan.comm_tasks.empty() ? 0 : a->num_comm_sm;
         const int grid = a->num_comp_sm + comm;
         profile_mark(B2A_KERNEL_BWD, false, stream);
-        bwd_kernel<<<grid, kBwdThreads, kRingBwdSmemBytes, stream>>>(map_q, map_k, map_v, map_do, p);
+        bwd_kernel<false><<<grid, kBwdThreads, kRingBwdSmemBytes, stream>>>(map_q, map_k, map_v, map_do, p);
         profile_mark(B2A_KERNEL_BWD, true, stream);
         B2A_CUDA_OK(cudaGetLastError());
 

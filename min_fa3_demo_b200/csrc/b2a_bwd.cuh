@@ -41,6 +41,7 @@ constexpr uint32_t kBwdExpPolyMask = B2A_BWD_EXP_POLY_MASK;
 constexpr int kBwdStages = 2;          // Q ring stages (with their LSE2 / D vectors)
 constexpr int kDoStages = 1;           // dO is single-buffered: it lives only from dP(t) to dV(t)
 constexpr uint32_t kDqBarrier = 1;          // named barrier of the dQ warpgroup
+constexpr int kBwdMaxSplits = 16;
 constexpr uint32_t kDqChunkBytes = 16384;   // 32 dQ columns x 128 rows fp32: one bulk reduction
 constexpr uint32_t kRowVecBytes = kTileM * 4;   // 128 fp32 (LSE2 or D of one query tile)
 
@@ -73,6 +74,13 @@ struct BwdParams {
     int sg_heads;      // key/value heads per scheduling supergroup (1..heads_k)
     int batch_minor;   // BSHD: hand out work key block major, batch element minor (deterministic mode)
     int padded_q;                  // padded query rows per head (multiple of 128)
+    // Step split (fixed-length calls): behind the first whole_items, an item with more than split_steps steps is cut
+    // into up to max_splits pieces that different CTAs compute and bwd_combine_kernel adds up in fp32.
+    // bwd_kernel<false> does not look at these.
+    int max_splits;
+    int whole_items;
+    int split_steps;
+    float4* split_part;            // [items that may be cut][max_splits][dV, dK][32][128]
     float scale;
     float scale_log2;
     uint32_t timeout_ns;
@@ -119,6 +127,10 @@ struct BwdWork {
     int diag_tile;
     int owner;         // ring mode: rank that owns the K/V block
     int owner_block;   // ring mode: 128-row block index inside the owner's slice
+    int t0, t1;        // steps [t0, t1) of the item's (query head, query tile) sequence
+    int splits;        // pieces of the item (1: not cut, 0: a piece that the item does not need)
+    int split;         // which piece this is
+    int item;          // number of the item among those that may be cut
 };
 
 // Query tile of step t (within one head): document-local first row and whether it is the
@@ -139,7 +151,7 @@ __host__ __device__ __forceinline__ int bwd_padded_begin(int cu_begin, int doc) 
     return ((cu_begin + 127) / 128) * 128 + 256 * doc;
 }
 
-__device__ __forceinline__ BwdWork bwd_decode_work(const BwdParams& p, int w) {
+__device__ __forceinline__ BwdWork bwd_decode_item(const BwdParams& p, int w) {
     BwdWork wk;
     // Work order: key/value heads are taken `sg_heads` at a time ("supergroup", sized by the host
     // so that the dQ accumulator rows being added to stay within L2); inside a supergroup the
@@ -254,6 +266,36 @@ __device__ __forceinline__ BwdWork bwd_decode_work(const BwdParams& p, int w) {
     wk.first0 = first;
     wk.count0 = m_tiles - first;
     wk.k_row = wk.k_begin + wk.n0;
+    return wk;
+}
+
+template <bool kSplit>
+__device__ __forceinline__ BwdWork bwd_decode_work(const BwdParams& p, int w) {
+    const bool cut = kSplit && w >= p.whole_items;
+    int item = 0, split = 0;
+    if (cut) {
+        const int c = w - p.whole_items;
+        item = c / p.max_splits;
+        split = c - item * p.max_splits;
+        w = p.whole_items + item;
+    }
+    BwdWork wk = bwd_decode_item(p, w);
+    const int steps = (wk.count0 + wk.count1) * (p.heads_q / p.heads_k);
+    wk.t0 = 0;
+    wk.t1 = steps;
+    wk.splits = 1;
+    wk.split = split;
+    wk.item = item;
+    if (cut) {
+        wk.splits = min(p.max_splits, max(1, (steps + p.split_steps - 1) / p.split_steps));
+        if (split >= wk.splits) {
+            wk.splits = 0;
+            wk.t1 = 0;
+        } else {
+            wk.t0 = steps * split / wk.splits;
+            wk.t1 = steps * (split + 1) / wk.splits;
+        }
+    }
     return wk;
 }
 
@@ -372,6 +414,9 @@ __device__ __forceinline__ void bwd_ring_copy_role(const BwdParams& p, BwdShared
     }
 }
 
+// kSplit: some items are cut along their steps.  A kernel of its own, because carrying the cut through the step loop costs
+// registers that the uncut one does not have to spare.
+template <bool kSplit>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
            const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -432,8 +477,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 384;
 
     WaitCtx wctx{smem_u32(&sh.abort_flag), p.status, p.timeout_ns};
-    const int total_work =
-        (p.cu_seqlens_q == nullptr ? p.num_entries_host : *p.num_entries_dev) * p.heads_k;
+    int total_work = (p.cu_seqlens_q == nullptr ? p.num_entries_host : *p.num_entries_dev) * p.heads_k;
+    if (kSplit) total_work += (total_work - p.whole_items) * (p.max_splits - 1);
     const int group = p.heads_q / p.heads_k;
 
     // Copy CTAs (ring mode) first pull the other ranks' K/V blocks into the local arena.
@@ -468,10 +513,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 w = __shfl_sync(0xFFFFFFFFu, w, 0);
                 if (lane == 0) mbar_arrive(smem_u32(&sh.sched_full[slot]));
                 if (w < 0) break;
-                const BwdWork wk = bwd_decode_work(p, w);
+                const BwdWork wk = bwd_decode_work<kSplit>(p, w);
                 const int per_head = wk.count0 + wk.count1;
-                const int steps = per_head * group;
-                if (steps == 0) continue;
+                if (wk.t0 == wk.t1) continue;
                 ok = mbar_wait(wctx, smem_u32(&sh.kv_empty), (item_cnt & 1u) ^ 1u, 2);
                 if (!ok) break;
                 ++item_cnt;
@@ -489,7 +533,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                     tma_load_3d(smem_u32(&sh.v[0]), &map_v, bar, 0, wk.head_k, row);
                     tma_load_3d(smem_u32(&sh.v[0]) + kHalfTileBytes, &map_v, bar, 64, wk.head_k, row);
                 }
-                for (int t = 0; t < steps && ok; ++t) {
+                for (int t = wk.t0; t < wk.t1 && ok; ++t) {
                     const int hq = wk.head_k * group + t / per_head;
                     bool diag;
                     const int q_local = bwd_step_row(wk, t % per_head, &diag);
@@ -559,9 +603,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&sh.sched_empty[slot]));
                 if (w < 0) break;
-                const BwdWork wk = bwd_decode_work(p, w);
-                const int steps = (wk.count0 + wk.count1) * group;
-                if (steps == 0) continue;
+                const BwdWork wk = bwd_decode_work<kSplit>(p, w);
+                if (wk.t0 == wk.t1) continue;
                 ok = mbar_wait(wctx, smem_u32(&sh.kv_full), item_cnt & 1u, 6);
                 if (!ok) break;
                 const uint32_t dkv_parity = (item_cnt & 1u) ^ 1u;
@@ -589,6 +632,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                     }
                     __syncwarp();
                 }
+                const int steps = wk.t1 - wk.t0;
                 for (int t = 0; t < steps && ok; ++t) {
                     const uint32_t stage = step_it % kBwdStages;
                     const uint32_t nstage = (step_it + 1) % kBwdStages;
@@ -695,12 +739,11 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 if (lane == 0) mbar_arrive(smem_u32(&sh.sched_empty[slot]));
                 if (w < 0) break;
                 if (p.dq_sem == nullptr) continue;
-                const BwdWork wk = bwd_decode_work(p, w);
+                const BwdWork wk = bwd_decode_work<kSplit>(p, w);
                 const int per_head = wk.count0 + wk.count1;
-                const int steps = per_head * group;
                 const int blk_index = wk.n0 / kTileN;
                 if (lane == 0) {
-                    for (int t = 0; t < steps && ok; ++t) {
+                    for (int t = wk.t0; t < wk.t1 && ok; ++t) {
                         const int hq = wk.head_k * group + t / per_head;
                         bool diag;
                         const int q_local = bwd_step_row(wk, t % per_head, &diag);
@@ -740,11 +783,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&sh.sched_empty[slot]));
             if (w < 0) break;
-            const BwdWork wk = bwd_decode_work(p, w);
+            const BwdWork wk = bwd_decode_work<kSplit>(p, w);
             const int per_head = wk.count0 + wk.count1;
-            const int steps = per_head * group;
             const int pad_tiles = p.padded_q / kTileM;
-            for (int t = 0; t < steps && ok; ++t) {
+            for (int t = wk.t0; t < wk.t1 && ok; ++t) {
                 const int hq = wk.head_k * group + t / per_head;
                 bool diag;
                 const int q_local = bwd_step_row(wk, t % per_head, &diag);
@@ -874,15 +916,16 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&sh.sched_empty[slot]));
             if (w < 0) break;
-            const BwdWork wk = bwd_decode_work(p, w);
+            const BwdWork wk = bwd_decode_work<kSplit>(p, w);
+            if (kSplit && wk.splits == 0) continue;
             const int per_head = wk.count0 + wk.count1;
-            const int steps = per_head * group;
+            const int steps = wk.t1 - wk.t0;
             const bool ring = p.ring_docs != nullptr;
             const int kv_row = wk.n0 + i_row;
             const bool kv_valid = kv_row < wk.k_len;
             const int shift = wk.k_len - wk.q_len;     // key c visible to query r iff c <= r + shift
 
-            for (int t = 0; t < steps && ok; ++t) {
+            for (int t = wk.t0; t < wk.t1 && ok; ++t) {
                 bool diag;
                 const int q_local = bwd_step_row(wk, t % per_head, &diag);
                 const uint32_t stage = step_it % kBwdStages;
@@ -1018,6 +1061,25 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 tc_fence_after_sync();
             }
             const uint32_t acc_tmem = tmem_base + lane_base + (wg == 0 ? kColDV : kColDK);
+            if (kSplit && wk.splits > 1) {
+                // Every piece stores its fp32 sums; bwd_combine_kernel adds them up.
+                float4* part = p.split_part +
+                               ((static_cast<long long>(wk.item) * p.max_splits + wk.split) * 2 + wg) * (32 * kTileM) + i_row;
+#pragma unroll 1
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t v[32];
+                    tmem_ld_x32(acc_tmem + c * 32, v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        part[(c * 8 + i) * kTileM] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                                                 __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+                    }
+                }
+                tc_fence_before_sync();
+                mbar_arrive(smem_u32(&sh.dkv_empty));
+                continue;
+            }
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 uint32_t v[32];

@@ -229,8 +229,7 @@ def _call_bwd(dout, q, k, v, out, lse, dq, dk, dv, *, cu_q, cu_k, batch, seqlen_
     args.grid_blocks = 0
     args.softmax_scale = 0.0
     with torch.cuda.device(q.device):
-        nbytes = lib.b2a_bwd_workspace_bytes(batch, total_q, total_k, heads_q, heads_k,
-                                             0 if cu_q is None else 1)
+        nbytes = lib.b2a_bwd_scratch_bytes(ctypes.byref(args))
         ws = _workspace(nbytes, q.device)
         args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
         _cabi.check(lib.b2a_bwd(ctypes.byref(args), _stream_ptr(q.device)))

@@ -3,10 +3,14 @@ against the fp32 autograd oracle and the reference's golden fixtures.  Acceptanc
 gradient within 2x the max-abs error of a bf16 PyTorch attention against the oracle."""
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 
 import min_fa3_op
+from min_fa3_demo_b200 import _cabi
+from min_fa3_demo_b200 import min_fa3_op as min_fa3_op_impl
 from conftest import from_bf16_bits, load_golden
 from gpu_util import assert_lse, assert_within, bound, make_bshd, make_varlen, varlen_bf16_errors
 from oracle import attention_oracle as orc
@@ -40,6 +44,46 @@ def test_bshd_backward_vs_oracle(b, s, qh, kvh, causal):
     assert_within("dQ", dq, rq, e["dq"])
     assert_within("dK", dk, rk, e["dk"])
     assert_within("dV", dv, rv, e["dv"])
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("b,sq,sk,qh,kvh,causal", [
+    (1, 256, 256, 8, 2, True),        # 4 key blocks of 8 and 4 steps
+    (1, 2000, 130, 2, 2, False),      # two key blocks, the second with two rows; 16 steps each
+    (1, 1000, 1000, 6, 2, True),      # groups of 3
+    (1, 300, 1500, 32, 1, True),      # one group of all heads; most key blocks are seen by all query tiles
+    (1, 700, 300, 4, 1, True),        # query tiles that see no key
+    (3, 1300, 1300, 20, 20, False),   # two full rounds of items and a rest, which alone is cut
+])
+def test_bshd_backward_cut_items(b, sq, sk, qh, kvh, causal, deterministic):
+    q, k, v, dout = make_bshd(17 + sq, b, sq, qh, kvh, sk=sk)
+    out, lse, (dq, dk, dv) = fwd_bwd_bshd(q, k, v, dout, causal, deterministic=deterministic)
+    min_fa3_op_impl.check_last_status("backward")
+    rq, rk, rv = orc.bshd_backward(q, k, v, dout, causal)
+    e = orc.bf16_attention_error(q, k, v, causal, dout)
+    assert_within("dQ", dq, rq, e["dq"])
+    assert_within("dK", dk, rk, e["dk"])
+    assert_within("dV", dv, rv, e["dv"])
+    # The pieces are added up in a fixed order, whichever CTA comes last.
+    dq2, dk2, dv2 = min_fa3_op.backward(dout.cuda(), q.cuda(), k.cuda(), v.cuda(), out, lse, causal,
+                                        deterministic=deterministic)
+    assert torch.equal(dk, dk2) and torch.equal(dv, dv2)
+    assert not deterministic or torch.equal(dq, dq2)
+    # The plain workspace is enough for the same call, without cutting the items.
+    lib = _cabi.load()
+    a = _cabi.BwdArgs()
+    held = [t.cuda() for t in (dout, q, k, v)] + [out, lse] + [torch.empty_like(t) for t in (dq, dk, dv)]
+    a.dout, a.q, a.k, a.v, a.out, a.lse, a.dq, a.dk, a.dv = (t.data_ptr() for t in held)
+    a.batch, a.seqlen_q, a.seqlen_k, a.total_q, a.total_k = b, sq, sk, b * sq, b * sk
+    a.heads_q, a.heads_k, a.head_dim, a.is_causal, a.deterministic = qh, kvh, 128, int(causal), int(deterministic)
+    plain = lib.b2a_bwd_workspace_bytes(b, b * sq, b * sk, qh, kvh, 0)
+    assert lib.b2a_bwd_scratch_bytes(ctypes.byref(a)) >= plain
+    ws = torch.empty(plain, dtype=torch.uint8, device="cuda")
+    a.workspace, a.workspace_bytes = ws.data_ptr(), plain
+    _cabi.check(lib.b2a_bwd(ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    for name, ours, ref in zip(("dq", "dk", "dv"), held[-3:], (rq, rk, rv)):
+        assert_within(f"{name} (plain workspace)", ours, ref, e[name])
 
 
 @pytest.mark.parametrize("sq,sk", [(256, 512), (300, 200)])
