@@ -30,3 +30,19 @@ def test_cpu_tensors_are_rejected():
     cu = torch.tensor([0, 128], dtype=torch.int32)
     with pytest.raises(RuntimeError, match="no CPU implementation"):
         ag.attention_varlen(q[0], q[0], q[0], cu, cu, 128, 128, True)
+
+
+def test_lookers_on_still_see_the_operators():
+    # Meta and fake tensors, tracers and dispatch modes go through the operators as before; only plain CUDA calls
+    # pass them by.
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.fx.experimental.proxy_tensor import make_fx
+    meta = torch.empty(1, 128, 4, 128, dtype=torch.bfloat16, device="meta", requires_grad=True)
+    out = ag.attention(meta, meta, meta, True)
+    assert out.device.type == "meta" and out.shape == meta.shape
+    assert torch.autograd.grad(out, meta, torch.empty_like(out))[0].shape == meta.shape
+    with FakeTensorMode():
+        q = torch.empty(1, 128, 4, 128, dtype=torch.bfloat16, device="meta")
+        assert not ag._plain_call(q)
+        graph = make_fx(lambda t: ag.attention(t, t, t, True))(q).graph
+    assert any(n.target is torch.ops.b200attn.fwd.default for n in graph.nodes)
