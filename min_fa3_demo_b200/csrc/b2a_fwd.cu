@@ -94,7 +94,7 @@ FwdSplit plan_fwd_split(const b2a_fwd_args& a, int ctas) {
     const size_t parts = static_cast<size_t>(cut) * best * s.tiles;
     s.stat_bytes = align_up(parts * s.rows * sizeof(float2), 256);
     s.o_bytes = align_up(parts * s.rows * kHeadDim * sizeof(float), 256);
-    return s.total() > (256ull << 20) ? FwdSplit{} : s;
+    return s.total() > (128ull << 20) ? FwdSplit{} : s;   // the caller's thread keeps the scratch of its latest call
 }
 
 // ---------------------------------------------------------------------------------------
