@@ -97,6 +97,10 @@ struct BwdSplit {
 // that can cut spills a little, and its steps take 1 to 2 % longer.  Measured (us, whole backward, not cut / cut): 2 x
 // 1,024 causal, 16 over 4 heads: 100 / 80; 1 x 4,096 causal, 8 over 2: 376 / 195; 1 x 2,048, 8 over 1: 305 / 85; 2 x
 // 3,001, 32 heads, the last of eleven rounds cut, which this leaves alone: 820 / 830.
+// Items below kBwdMinCutSteps steps are never cut: little is gained (1 x 512 causal, 32 over 8 heads, 16 steps: 63 / 58),
+// and the last bits of short calls stay the same however a batch is divided into calls.
+constexpr int kBwdMinCutSteps = 24;
+
 BwdSplit plan_bwd_split(const b2a_bwd_args& a, int ctas) {
     BwdSplit s;
     if (a.cu_seqlens_q != nullptr) return s;
@@ -105,7 +109,7 @@ BwdSplit plan_bwd_split(const b2a_bwd_args& a, int ctas) {
     const int group = a.heads_q / a.heads_k;
     const int tiles = (a.seqlen_q + kTileM - 1) / kTileM;
     const long long n = static_cast<long long>(tiles) * group;   // steps of the longest item
-    if (n < 4 || items >= 16ll * ctas) return s;
+    if (n < kBwdMinCutSteps || items >= 16ll * ctas) return s;
     double mean = 0;
     for (long long i = 0; i < nnb; ++i) {
         const long long first_row = std::max<long long>(0, i * kTileN + a.seqlen_q - a.seqlen_k);

@@ -12,7 +12,9 @@ starts as soon as q, k, v have arrived (dout follows during the forward) and ``o
 while the backward runs.  The head subset of a ``[B, S, H, 128]`` host tensor is strided; it is
 moved with the library's 2-D copy (``b2a_copy_2d``) straight between the pinned tensor and a
 contiguous device buffer.  Results equal one call over the whole problem bit for bit except dq,
-whose fp32 accumulation order is not fixed (every head sees the same kernels and data).
+whose fp32 accumulation order is not fixed (every head sees the same kernels and data).  The last
+bits can differ as well where a call has so few work items that it cuts them (``plan_fwd_split``,
+``plan_bwd_split``): how many items there are depends on how the problem is divided into chunks.
 """
 
 from __future__ import annotations

@@ -48,12 +48,12 @@ def test_bshd_backward_vs_oracle(b, s, qh, kvh, causal):
 
 @pytest.mark.parametrize("deterministic", [False, True])
 @pytest.mark.parametrize("b,sq,sk,qh,kvh,causal", [
-    (1, 256, 256, 8, 2, True),        # 4 key blocks of 8 and 4 steps
-    (1, 2000, 130, 2, 2, False),      # two key blocks, the second with two rows; 16 steps each
-    (1, 1000, 1000, 6, 2, True),      # groups of 3
+    (1, 256, 256, 8, 2, True),        # too short to be cut
+    (1, 4000, 130, 2, 2, False),      # two key blocks, the second with two rows; 32 steps each
+    (1, 1000, 1000, 6, 2, True),      # groups of 3, 24 steps: the shortest that is cut
     (1, 300, 1500, 32, 1, True),      # one group of all heads; most key blocks are seen by all query tiles
     (1, 700, 300, 4, 1, True),        # query tiles that see no key
-    (3, 1300, 1300, 20, 20, False),   # two full rounds of items and a rest, which alone is cut
+    (1, 3100, 900, 20, 20, False),    # a full round of items and a rest, which alone is cut
 ])
 def test_bshd_backward_cut_items(b, sq, sk, qh, kvh, causal, deterministic):
     q, k, v, dout = make_bshd(17 + sq, b, sq, qh, kvh, sk=sk)
