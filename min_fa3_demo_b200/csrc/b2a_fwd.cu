@@ -124,18 +124,26 @@ fwd_combine_kernel(const FwdParams p) {
     const long long at = static_cast<long long>(item) * p.max_splits * step + x * p.split_rows + first;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int head0 = fwd_tile_head(wk, x);
+    // What the uncut kernel leaves of NaN and infinities is left here as well: a sum that is NaN or empty gives the norm 0
+    // (O * 0 keeps NaN) and -inf for LSE, and a piece whose weight is 0 is multiplied by it like the others.  Only a
+    // piece without a block for this tile is skipped (sum -1, weight -1): its O was never stored.
     if (warp == 0 && lane < rows) {
         float m = -INFINITY, l = 0.f;
         for (int i = 0; i < wk.splits; ++i) m = fmaxf(m, p.split_stat[at + i * step + lane].x);
         for (int i = 0; i < wk.splits; ++i) {
             const float2 st = p.split_stat[at + i * step + lane];
-            const float f = st.x == -INFINITY ? 0.f : fast_exp2((st.x - m) * p.scale_log2);   // 0: saw no key
-            weight[i][lane] = f;
-            l = fmaf(st.y, f, l);
+            // -inf: the row saw no key here (or only NaN, which its sum carries).  m itself may be infinite.
+            const float f = st.x == -INFINITY ? 0.f : st.x == m ? 1.f : fast_exp2((st.x - m) * p.scale_log2);
+            const bool stored = st.y != -1.f;
+            weight[i][lane] = stored ? f : -1.f;
+            if (stored) l = fmaf(st.y, f, l);
         }
         const bool seen = l > 0.f && m != -INFINITY;
         const float norm = seen ? 1.f / l : 0.f;
-        for (int i = 0; i < wk.splits; ++i) weight[i][lane] *= norm;
+        for (int i = 0; i < wk.splits; ++i) {
+            const float f = weight[i][lane];
+            if (f != -1.f) weight[i][lane] = f * norm;
+        }
         const int tr = first + lane;
         p.lse[wk.lse_base + static_cast<long long>(head0 - wk.head + (tr & ((1 << wk.shift) - 1))) * p.lse_head_stride + row0 +
               (tr >> wk.shift)] = seen ? (m * p.scale_log2 + fast_log2(l)) * kLn2 : -INFINITY;
@@ -150,13 +158,13 @@ fwd_combine_kernel(const FwdParams p) {
 #pragma unroll 2
         for (int i = 0; i < wk.splits; ++i) {
             const float f = weight[i][lane];
+            if (f == -1.f) continue;
             const float4* o = p.split_o + base + i * step * 32;
             float4 v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) v[u] = __ldcs(o + static_cast<long long>(warp * 4 + u) * p.split_rows);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                if (f == 0.f) v[u] = make_float4(0.f, 0.f, 0.f, 0.f);   // perhaps never stored
                 acc[u].x = fmaf(v[u].x, f, acc[u].x);
                 acc[u].y = fmaf(v[u].y, f, acc[u].y);
                 acc[u].z = fmaf(v[u].z, f, acc[u].z);

@@ -86,7 +86,8 @@ struct FwdParams {
     int split_blocks;
     int split_tiles;             // row tiles of an item that hold rows (1 or 2)
     int split_rows;              // rows of a tile that hold any (at most 128)
-    float2* split_stat;          // [items * max_splits * split_tiles][split_rows] (row maximum, row sum)
+    float2* split_stat;          // [items * max_splits * split_tiles][split_rows] (row maximum, row sum); sum -1: the
+                                 // piece has no block for this tile, its O is not stored
     float4* split_o;             // [items * max_splits * split_tiles][32][split_rows] unnormalised O
     float scale;                 // softmax scale
     float scale_log2;            // scale * log2(e)
@@ -975,7 +976,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 // pieces up.
                 const int rows = p.split_rows;
                 const long long at = (static_cast<long long>(wk.item * p.max_splits + wk.split) * p.split_tiles + x) * rows + r;
-                if (row_valid) p.split_stat[at] = make_float2(m_used, l);
+                if (row_valid) p.split_stat[at] = make_float2(m_used, nblk > 0 ? l : -1.f);
                 float4* dst = p.split_o + (at - r) * 32 + r;
 #pragma unroll
                 for (int c = 0; c < 4 && nblk > 0; ++c) {

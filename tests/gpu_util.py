@@ -1,10 +1,12 @@
 """Helpers for the GPU parity tests: inputs, tolerances, per-document comparison."""
 from __future__ import annotations
 
+import ctypes
 from typing import Sequence
 
 import torch
 
+from min_fa3_demo_b200 import _cabi
 from oracle import attention_oracle as orc
 
 LSE_ATOL = 1e-3            # absolute LSE tolerance of the acceptance rule
@@ -32,6 +34,26 @@ def make_varlen(seed: int, lengths: Sequence[int], qh: int, kvh: int):
     dout = torch.randn(total, qh, 128, generator=gen).to(torch.bfloat16)
     cu = torch.tensor([0, *torch.tensor(list(lengths)).cumsum(0).tolist()], dtype=torch.int32)
     return q, k, v, dout, cu
+
+
+def plain_workspace_forward(q, k, v, causal):
+    """``b2a_fwd`` on CUDA tensors with ``b2a_fwd_workspace_bytes`` of scratch, i.e. never cut along the keys.
+    Returns (out, lse, whether ``b2a_fwd_scratch_bytes`` asks for more, as it does where the call would be cut)."""
+    lib = _cabi.load()
+    b, sq, qh, _ = q.shape
+    out, lse = torch.empty_like(q), torch.empty(b, qh, sq, dtype=torch.float32, device=q.device)
+    a = _cabi.FwdArgs()
+    a.q, a.k, a.v, a.out, a.lse = (t.data_ptr() for t in (q, k, v, out, lse))
+    a.batch, a.seqlen_q, a.seqlen_k, a.total_q, a.total_k = b, sq, k.size(1), b * sq, b * k.size(1)
+    a.heads_q, a.heads_k, a.head_dim, a.is_causal = qh, k.size(2), 128, int(causal)
+    plain = lib.b2a_fwd_workspace_bytes(b, b * sq, 0)
+    full = lib.b2a_fwd_scratch_bytes(ctypes.byref(a))
+    assert full >= plain
+    ws = torch.empty(plain, dtype=torch.uint8, device=q.device)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), plain
+    _cabi.check(lib.b2a_fwd(ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    return out, lse, full > plain
 
 
 def bound(e_bf16: float) -> float:

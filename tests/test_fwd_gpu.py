@@ -3,16 +3,14 @@ oracle and the reference's golden fixtures.  Acceptance: O within 2x the max-abs
 bf16 PyTorch attention against the fp32 oracle, LSE within 1e-3 absolute."""
 from __future__ import annotations
 
-import ctypes
-
 import pytest
 import torch
 
 import min_fa3_op
-from min_fa3_demo_b200 import _cabi
 from min_fa3_demo_b200 import min_fa3_op as min_fa3_op_impl
 from conftest import from_bf16_bits, load_golden
-from gpu_util import (assert_lse, assert_within, bound, make_bshd, make_varlen, varlen_bf16_errors)
+from gpu_util import (assert_lse, assert_within, bound, make_bshd, make_varlen, plain_workspace_forward,
+                      varlen_bf16_errors)
 from oracle import attention_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -81,21 +79,36 @@ def test_bshd_forward_packed_rows_and_key_pieces(b, sq, sk, qh, kvh, causal):
     assert_within("O", out, ref_out, e)
     assert_lse(lse, ref_lse)
     # The plain workspace is enough for the same call, without cutting the keys.
-    lib = _cabi.load()
-    a = _cabi.FwdArgs()
-    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
-    out2, lse2 = torch.empty_like(qd), torch.empty_like(lse)
-    a.q, a.k, a.v, a.out, a.lse = (t.data_ptr() for t in (qd, kd, vd, out2, lse2))
-    a.batch, a.seqlen_q, a.seqlen_k, a.total_q, a.total_k = b, sq, sk, b * sq, b * sk
-    a.heads_q, a.heads_k, a.head_dim, a.is_causal = qh, kvh, 128, int(causal)
-    plain = lib.b2a_fwd_workspace_bytes(b, b * sq, 0)
-    assert lib.b2a_fwd_scratch_bytes(ctypes.byref(a)) >= plain
-    ws = torch.empty(plain, dtype=torch.uint8, device="cuda")
-    a.workspace, a.workspace_bytes = ws.data_ptr(), plain
-    _cabi.check(lib.b2a_fwd(ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
-    torch.cuda.synchronize()
+    out2, lse2, _ = plain_workspace_forward(q.cuda(), k.cuda(), v.cuda(), causal)
     assert_within("O (plain workspace)", out2, ref_out, e)
     assert_lse(lse2, ref_lse)
+
+
+@pytest.mark.parametrize("b,sq,sk,qh,kvh,causal", [
+    (2, 1, 4001, 8, 2, True),         # eight pieces
+    (1, 300, 4096, 4, 4, False),      # two tiles, the second with 44 rows
+    (1, 2048, 2048, 8, 2, True),      # items of one piece and pieces without a block for the first tile
+])
+def test_key_pieces_keep_nan_and_infinities(b, sq, sk, qh, kvh, causal):
+    # A NaN or an infinity shows in the same places whether the keys are cut or not: one in a query row, in a key (none of
+    # those whose exponential is the polynomial, which clamps NaN in both kernels) or in a value.
+    q, k, v, _ = (t.cuda() for t in make_bshd(5 + sq, b, sq, qh, kvh, sk=sk))
+    for name, row, value in (("q", sq // 2, float("nan")), ("k", 5, float("nan")), ("k", sk // 2 + 1, float("nan")),
+                             ("k", sk - 1, float("nan")), ("v", 5, float("nan")), ("v", sk - 1, float("inf"))):
+        bad = {"q": q, "k": k, "v": v}
+        bad[name] = bad[name].clone()
+        bad[name][0, row, 0, 77] = value
+        out, lse = run_bshd(bad["q"], bad["k"], bad["v"], causal)
+        plain_out, plain_lse, cut = plain_workspace_forward(bad["q"], bad["k"], bad["v"], causal)
+        if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+            assert cut
+        where = f"{name}[{row}] = {value}"
+        assert not torch.isfinite(plain_out).all(), where
+        assert torch.equal(torch.isnan(out), torch.isnan(plain_out)), where
+        assert torch.equal(torch.isposinf(out), torch.isposinf(plain_out)), where
+        assert torch.equal(torch.isneginf(out), torch.isneginf(plain_out)), where
+        assert torch.equal(torch.isnan(lse), torch.isnan(plain_lse)), where
+        assert torch.equal(torch.isneginf(lse), torch.isneginf(plain_lse)), where
 
 
 @pytest.mark.parametrize("tag,causal", [("full", False), ("causal", True)])
