@@ -67,12 +67,19 @@ def _(dout, q, k, v, out, lse, is_causal, deterministic):
     return torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
 
 
+def _plain_tensor(t: torch.Tensor) -> bool:
+    return type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda
+
+
 def _plain_call(*tensors: torch.Tensor) -> bool:
     """Whether nothing looks on that has to see an operator: plain CUDA tensors, no compiler, no dispatch or function mode
-    (fake tensors, tracers, a user's own) and no functorch transform.  The operators' bodies can then be called as they
-    are; going through the dispatcher costs the host about 15 us a call, a fifth of a small training step."""
-    return (all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda for t in tensors)
-            and not torch.compiler.is_compiling()
+    (fake tensors, tracers, a user's own), no functorch transform, and no graph being recorded.  The operators' bodies can
+    then be called as they are; going through the dispatcher costs the host about 15 us a call, a fifth of a small
+    training step.  Grad mode is off in ``forward`` and in an ordinary ``backward``; with ``create_graph=True`` it is on,
+    and it is the operator that then refuses to be differentiated."""
+    return (not torch.compiler.is_compiling()
+            and not torch.is_grad_enabled()
+            and all(map(_plain_tensor, tensors))
             and _get_current_dispatch_mode() is None
             and torch._C._len_torch_function_stack() == 0
             and torch._C._functorch.peek_interpreter_stack() is None)

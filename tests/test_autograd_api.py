@@ -46,3 +46,33 @@ def test_lookers_on_still_see_the_operators():
         assert not ag._plain_call(q)
         graph = make_fx(lambda t: ag.attention(t, t, t, True))(q).graph
     assert any(n.target is torch.ops.b200attn.fwd.default for n in graph.nodes)
+
+
+def _stand_ins(monkeypatch):
+    """Lets CPU tensors pass for CUDA ones, with cheap functions in the kernels' place; records direct calls."""
+    direct = []
+    monkeypatch.setattr(ag, "_require_cuda", lambda t, name: None)
+    monkeypatch.setattr(ag, "_plain_tensor", lambda t: type(t) in (torch.Tensor, torch.nn.Parameter))
+    monkeypatch.setattr(ag._op, "forward", lambda q, k, v, causal, return_lse: (q * 2, q.new_zeros(
+        (q.size(0), q.size(2), q.size(1)), dtype=torch.float32)))
+    monkeypatch.setattr(ag._op, "backward", lambda dout, q, k, v, out, lse, causal, deterministic: (
+        dout * 2, torch.zeros_like(k), torch.zeros_like(v)))
+    for name in ("_fwd", "_bwd"):
+        def body(*args, _body=getattr(ag, name), _name=name):
+            direct.append(_name)
+            return _body(*args)
+        monkeypatch.setattr(ag, name, body)
+    return direct
+
+
+def test_differentiating_a_gradient_is_refused(monkeypatch):
+    direct = _stand_ins(monkeypatch)
+    q, k, v = (torch.ones(1, 4, 2, 128, dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
+    out = ag.attention(q, k, v, True)
+    out.sum().backward()
+    assert direct == ["_fwd", "_bwd"]                   # an ordinary step passes the operators by
+    assert torch.equal(q.grad, torch.full_like(q, 2))
+    out = ag.attention(q, k, v, True)
+    grad, = torch.autograd.grad(out.sum(), q, create_graph=True)
+    with pytest.raises(RuntimeError, match="no autograd formula"):
+        (out.sum() + grad.square().sum()).backward()

@@ -53,3 +53,11 @@ def test_operators_compose_with_other_autograd_nodes():
     out = ag.attention(qc @ w, k.cuda(), v.cuda(), True)
     out.float().square().mean().backward()
     assert w.grad is not None and torch.isfinite(w.grad.float()).all() and w.grad.float().abs().sum() > 0
+
+
+def test_differentiating_a_gradient_is_refused():
+    q, k, v, _ = (t.cuda().requires_grad_() for t in make_bshd(34, 1, 200, 4, 2))
+    out = ag.attention(q, k, v, True)
+    grad, = torch.autograd.grad(out.float().sum(), q, create_graph=True)
+    with pytest.raises(RuntimeError, match="no autograd formula"):
+        (out.float().sum() + grad.float().square().sum()).backward()
