@@ -68,7 +68,9 @@ def _(dout, q, k, v, out, lse, is_causal, deterministic):
 
 
 def _plain_tensor(t: torch.Tensor) -> bool:
-    return type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda
+    # A lazily negated view's memory holds the values before the negation, and a zero tensor has no memory; the dispatcher
+    # puts proper values in both before it calls a kernel.
+    return type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and not t.is_neg() and not t._is_zerotensor()
 
 
 def _plain_call(*tensors: torch.Tensor) -> bool:

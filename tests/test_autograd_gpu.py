@@ -61,3 +61,17 @@ def test_differentiating_a_gradient_is_refused():
     grad, = torch.autograd.grad(out.float().sum(), q, create_graph=True)
     with pytest.raises(RuntimeError, match="no autograd formula"):
         (out.float().sum() + grad.float().square().sum()).backward()
+
+
+def test_negated_views_and_zero_tensors():
+    q, k, v, dout = (t.cuda() for t in make_bshd(35, 1, 200, 4, 2))
+    k.requires_grad_()
+    neg = torch._neg_view
+    assert neg(q).is_neg()
+    out = ag.attention(neg(q), k, v, True, deterministic=True)
+    want = ag.attention(-q, k, v, True, deterministic=True)
+    assert torch.equal(out, want)
+    dk, = torch.autograd.grad(out, k, neg(dout), retain_graph=True)
+    assert torch.equal(dk, torch.autograd.grad(want, k, -dout)[0])
+    zero = torch._efficientzerotensor(out.shape, dtype=out.dtype, device=out.device)
+    assert not torch.autograd.grad(out, k, zero)[0].any()
