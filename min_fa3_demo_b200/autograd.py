@@ -25,7 +25,6 @@ from __future__ import annotations
 from typing import List, Optional, Sequence, Tuple
 
 import torch
-from torch.utils._python_dispatch import _get_current_dispatch_mode
 
 from . import min_fa3_op as _op
 
@@ -67,6 +66,21 @@ def _(dout, q, k, v, out, lse, is_causal, deterministic):
     return torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
 
 
+def _looker_checks():
+    """What tells whether a profiler, a dispatch mode, a function mode or a functorch transform looks on.  These functions are
+    torch's own and may go: ``None`` where this release lacks one, and every call then takes the operators."""
+    try:
+        from torch.utils._python_dispatch import _get_current_dispatch_mode
+        torch.Tensor._is_zerotensor
+        return (torch._C._autograd._profiler_enabled, _get_current_dispatch_mode, torch._C._len_torch_function_stack,
+                torch._C._functorch.peek_interpreter_stack)
+    except (ImportError, AttributeError):
+        return None
+
+
+_LOOKER_CHECKS = _looker_checks()
+
+
 def _plain_tensor(t: torch.Tensor) -> bool:
     # A lazily negated view's memory holds the values before the negation, and a zero tensor has no memory; the dispatcher
     # puts proper values in both before it calls a kernel.
@@ -74,17 +88,16 @@ def _plain_tensor(t: torch.Tensor) -> bool:
 
 
 def _plain_call(*tensors: torch.Tensor) -> bool:
-    """Whether nothing looks on that has to see an operator: plain CUDA tensors, no compiler, no dispatch or function mode
-    (fake tensors, tracers, a user's own), no functorch transform, and no graph being recorded.  The operators' bodies can
-    then be called as they are; going through the dispatcher costs the host about 15 us a call, a fifth of a small
-    training step.  Grad mode is off in ``forward`` and in an ordinary ``backward``; with ``create_graph=True`` it is on,
-    and it is the operator that then refuses to be differentiated."""
+    """Whether nothing looks on that has to see an operator: plain CUDA tensors, no compiler, no profiler, no dispatch or
+    function mode (fake tensors, tracers, a user's own), no functorch transform, and no graph being recorded.  The
+    operators' bodies can then be called as they are; going through the dispatcher costs the host about 15 us a call, a
+    fifth of a small training step.  Grad mode is off in ``forward`` and in an ordinary ``backward``; with
+    ``create_graph=True`` it is on, and it is the operator that then refuses to be differentiated."""
     return (not torch.compiler.is_compiling()
+            and _LOOKER_CHECKS is not None
             and not torch.is_grad_enabled()
             and all(map(_plain_tensor, tensors))
-            and _get_current_dispatch_mode() is None
-            and torch._C._len_torch_function_stack() == 0
-            and torch._C._functorch.peek_interpreter_stack() is None)
+            and not any(check() for check in _LOOKER_CHECKS))
 
 
 class _Attention(torch.autograd.Function):

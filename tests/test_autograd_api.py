@@ -32,22 +32,6 @@ def test_cpu_tensors_are_rejected():
         ag.attention_varlen(q[0], q[0], q[0], cu, cu, 128, 128, True)
 
 
-def test_lookers_on_still_see_the_operators():
-    # Meta and fake tensors, tracers and dispatch modes go through the operators as before; only plain CUDA calls
-    # pass them by.
-    from torch._subclasses.fake_tensor import FakeTensorMode
-    from torch.fx.experimental.proxy_tensor import make_fx
-    meta = torch.empty(1, 128, 4, 128, dtype=torch.bfloat16, device="meta", requires_grad=True)
-    out = ag.attention(meta, meta, meta, True)
-    assert out.device.type == "meta" and out.shape == meta.shape
-    assert torch.autograd.grad(out, meta, torch.empty_like(out))[0].shape == meta.shape
-    with FakeTensorMode():
-        q = torch.empty(1, 128, 4, 128, dtype=torch.bfloat16, device="meta")
-        assert not ag._plain_call(q)
-        graph = make_fx(lambda t: ag.attention(t, t, t, True))(q).graph
-    assert any(n.target is torch.ops.b200attn.fwd.default for n in graph.nodes)
-
-
 def _stand_ins(monkeypatch):
     """Lets CPU tensors pass for CUDA ones, with cheap functions in the kernels' place; records direct calls."""
     direct = []
@@ -76,3 +60,68 @@ def test_differentiating_a_gradient_is_refused(monkeypatch):
     grad, = torch.autograd.grad(out.sum(), q, create_graph=True)
     with pytest.raises(RuntimeError, match="no autograd formula"):
         (out.sum() + grad.square().sum()).backward()
+
+
+def test_lookers_on_still_see_the_operators(monkeypatch):
+    # Meta and fake tensors, tracers, dispatch and function modes and profilers see the operators; only plain CUDA calls
+    # pass them by.
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    meta = torch.empty(1, 128, 4, 128, dtype=torch.bfloat16, device="meta", requires_grad=True)
+    out = ag.attention(meta, meta, meta, True)
+    assert out.device.type == "meta" and out.shape == meta.shape
+    assert torch.autograd.grad(out, meta, torch.empty_like(out))[0].shape == meta.shape
+    with FakeTensorMode():
+        q = torch.empty(1, 128, 4, 128, dtype=torch.bfloat16, device="meta")
+        assert not ag._plain_call(q)
+        graph = make_fx(lambda t: ag.attention(t, t, t, True))(q).graph
+    assert any(n.target is torch.ops.b200attn.fwd.default for n in graph.nodes)
+
+    direct = _stand_ins(monkeypatch)
+    seen = []
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    def step():
+        q = torch.ones(1, 4, 2, 128, dtype=torch.bfloat16, requires_grad=True)
+        ag.attention(q, q, q, True).sum().backward()
+        assert torch.equal(q.grad, torch.full_like(q, 2))
+
+    with Dispatch():
+        step()
+    assert torch.ops.b200attn.fwd.default in seen and torch.ops.b200attn.bwd.default in seen
+    seen.clear()
+    with Function():
+        step()
+    assert torch.ops.b200attn.fwd in seen
+    assert direct in ([], ["_bwd"])                        # backward() runs inside the mode's handler, without the mode
+    direct.clear()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        step()
+    assert {"b200attn::fwd", "b200attn::bwd"} <= {e.key for e in prof.key_averages()}
+    graph = make_fx(lambda t: ag.attention(t, t, t, True))(torch.ones(1, 4, 2, 128, dtype=torch.bfloat16)).graph
+    assert any(n.target is torch.ops.b200attn.fwd.default for n in graph.nodes)
+    monkeypatch.setattr(ag, "_LOOKER_CHECKS", None)       # a torch without the checks
+    step()
+    assert direct == []
+
+
+@pytest.mark.parametrize("owner,name", [("torch.utils._python_dispatch", "_get_current_dispatch_mode"),
+                                        ("torch._C._functorch", "peek_interpreter_stack"),
+                                        ("torch._C", "_len_torch_function_stack"),
+                                        ("torch._C._autograd", "_profiler_enabled")])
+def test_a_torch_without_a_check_is_found_out(monkeypatch, owner, name):
+    import importlib
+    assert ag._looker_checks() is not None
+    monkeypatch.delattr(importlib.import_module(owner), name)
+    assert ag._looker_checks() is None
