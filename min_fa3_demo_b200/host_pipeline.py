@@ -11,10 +11,11 @@ and chunk ``c - 2`` is downloaded on a third (PCIe is full duplex); within a chu
 starts as soon as q, k, v have arrived (dout follows during the forward) and ``out`` goes back
 while the backward runs.  The head subset of a ``[B, S, H, 128]`` host tensor is strided; it is
 moved with the library's 2-D copy (``b2a_copy_2d``) straight between the pinned tensor and a
-contiguous device buffer.  Results equal one call over the whole problem bit for bit except dq,
-whose fp32 accumulation order is not fixed (every head sees the same kernels and data).  The last
-bits can differ as well where a call has so few work items that it cuts them (``plan_fwd_split``,
-``plan_bwd_split``): how many items there are depends on how the problem is divided into chunks.
+contiguous device buffer.  Every head sees the same kernels and data however the problem is divided:
+the chunks run uncut (``may_cut=False``), so out, dk and dv are bit for bit those of one uncut call
+over the whole problem, and dq differs by its fp32 accumulation order only, which is not fixed.  A
+direct call of ``forward`` / ``backward`` with too few work items for the GPU is cut, and then its
+last bits differ (rounding; see ``b2a_fwd_scratch_bytes``).
 """
 
 from __future__ import annotations
@@ -103,6 +104,22 @@ class HostPipeline:
                 raise ValueError(f"{name} must have shape {want[name]}, got {tuple(t.shape)}")
         return batch
 
+    def _sizes(self):
+        return dict(cu_q=None, cu_k=None, batch=1, seqlen_q=self.seqlen_q, seqlen_k=self.seqlen_k, heads_q=self.hq_c,
+                    heads_k=self.hk_c, may_cut=False)
+
+    def _forward(self, i, is_causal: bool):
+        out = torch.empty_like(i["q"])
+        lse = torch.empty((1, self.hq_c, self.seqlen_q), dtype=torch.float32, device=self.device)
+        ws = _op._call_fwd(i["q"], i["k"], i["v"], out, lse, is_causal=is_causal, **self._sizes())
+        _op._remember_workspace("forward", ws)
+        return out, lse
+
+    def _backward(self, i, o, out, lse, is_causal: bool) -> None:
+        ws = _op._call_bwd(i["dout"], i["q"], i["k"], i["v"], out, lse, o["dq"], o["dk"], o["dv"], is_causal=is_causal,
+                           deterministic=False, **self._sizes())
+        _op._remember_workspace("backward", ws)
+
     def run(self, host_in: Dict[str, torch.Tensor], host_out: Dict[str, torch.Tensor], is_causal: bool) -> None:
         batch = self._check(host_in, host_out)
         caller = torch.cuda.current_stream(self.device)
@@ -128,12 +145,11 @@ class HostPipeline:
                     self.s_compute.wait_event(self.ev_qkv[slot])
                     if reuse:
                         self.s_compute.wait_event(self.ev_downloaded[slot])   # outputs of chunk c - slots read
-                    out, lse = _op.forward(i["q"], i["k"], i["v"], is_causal, return_lse=True)
+                    out, lse = self._forward(i, is_causal)
                     o["out"].copy_(out)
                     self.ev_fwd[slot].record(self.s_compute)
                     self.s_compute.wait_event(self.ev_dout[slot])
-                    _op.backward(i["dout"], i["q"], i["k"], i["v"], out, lse, is_causal,
-                                 dq=o["dq"], dk=o["dk"], dv=o["dv"])
+                    self._backward(i, o, out, lse, is_causal)
                     self.ev_bwd[slot].record(self.s_compute)
                 self.s_out.wait_event(self.ev_fwd[slot])
                 self._copy(o["out"], host_out["out"], b, g, _D2H, self.s_out)    # overlaps the backward

@@ -180,9 +180,11 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads_q, heads_k,
-              is_causal, merge_running=False, grid_blocks=0, prefetch=None):
+              is_causal, merge_running=False, grid_blocks=0, prefetch=None, may_cut=True):
     """``prefetch``: optional ``(src_k_ptr, src_v_ptr, dst_k, dst_v, blocks)`` -- that many extra
-    CTAs of the launch copy ``dst_k.numel() * 2`` bytes from each source address first."""
+    CTAs of the launch copy ``dst_k.numel() * 2`` bytes from each source address first.
+    ``may_cut=False``: only the scratch of an uncut call, whose results do not depend on how many
+    other heads and batch elements the call has."""
     lib = _cabi.load()
     total_q = q.numel() // (heads_q * 128)
     total_k = k.numel() // (heads_k * 128)
@@ -204,7 +206,10 @@ def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads
         args.prefetch_bytes = dst_k.numel() * dst_k.element_size()
         args.prefetch_blocks = int(blocks)
     with torch.cuda.device(q.device):
-        nbytes = lib.b2a_fwd_scratch_bytes(ctypes.byref(args))
+        if may_cut:
+            nbytes = lib.b2a_fwd_scratch_bytes(ctypes.byref(args))
+        else:
+            nbytes = lib.b2a_fwd_workspace_bytes(batch, total_q, 0 if cu_q is None else 1)
         ws = _workspace(nbytes, q.device)
         args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
         _cabi.check(lib.b2a_fwd(ctypes.byref(args), _stream_ptr(q.device)))
@@ -212,7 +217,8 @@ def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads
 
 
 def _call_bwd(dout, q, k, v, out, lse, dq, dk, dv, *, cu_q, cu_k, batch, seqlen_q, seqlen_k,
-              heads_q, heads_k, is_causal, deterministic):
+              heads_q, heads_k, is_causal, deterministic, may_cut=True):
+    """``may_cut``: as in :func:`_call_fwd`."""
     lib = _cabi.load()
     total_q = q.numel() // (heads_q * 128)
     total_k = k.numel() // (heads_k * 128)
@@ -229,7 +235,11 @@ def _call_bwd(dout, q, k, v, out, lse, dq, dk, dv, *, cu_q, cu_k, batch, seqlen_
     args.grid_blocks = 0
     args.softmax_scale = 0.0
     with torch.cuda.device(q.device):
-        nbytes = lib.b2a_bwd_scratch_bytes(ctypes.byref(args))
+        if may_cut:
+            nbytes = lib.b2a_bwd_scratch_bytes(ctypes.byref(args))
+        else:
+            nbytes = lib.b2a_bwd_workspace_bytes(batch, total_q, total_k, heads_q, heads_k,
+                                                 0 if cu_q is None else 1)
         ws = _workspace(nbytes, q.device)
         args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
         _cabi.check(lib.b2a_bwd(ctypes.byref(args), _stream_ptr(q.device)))

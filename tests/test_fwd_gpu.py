@@ -9,7 +9,7 @@ import torch
 import min_fa3_op
 from min_fa3_demo_b200 import min_fa3_op as min_fa3_op_impl
 from conftest import from_bf16_bits, load_golden
-from gpu_util import (assert_lse, assert_within, bound, make_bshd, make_varlen, plain_workspace_forward,
+from gpu_util import (assert_cut, assert_lse, assert_within, bound, make_bshd, make_varlen, plain_workspace_forward,
                       varlen_bf16_errors)
 from oracle import attention_oracle as orc
 
@@ -79,7 +79,7 @@ def test_bshd_forward_packed_rows_and_key_pieces(b, sq, sk, qh, kvh, causal):
     assert_within("O", out, ref_out, e)
     assert_lse(lse, ref_lse)
     # The plain workspace is enough for the same call, without cutting the keys.
-    out2, lse2, _ = plain_workspace_forward(q.cuda(), k.cuda(), v.cuda(), causal)
+    out2, lse2 = plain_workspace_forward(q.cuda(), k.cuda(), v.cuda(), causal)
     assert_within("O (plain workspace)", out2, ref_out, e)
     assert_lse(lse2, ref_lse)
 
@@ -92,6 +92,7 @@ def test_bshd_forward_packed_rows_and_key_pieces(b, sq, sk, qh, kvh, causal):
 def test_key_pieces_keep_nan_and_infinities(b, sq, sk, qh, kvh, causal):
     # A NaN or an infinity shows in the same places whether the keys are cut or not: one in a query row, in a key (none of
     # those whose exponential is the polynomial, which clamps NaN in both kernels) or in a value.
+    assert_cut(True, "fwd", b, sq, sk, qh, kvh, causal)
     q, k, v, _ = (t.cuda() for t in make_bshd(5 + sq, b, sq, qh, kvh, sk=sk))
     for name, row, value in (("q", sq // 2, float("nan")), ("k", 5, float("nan")), ("k", sk // 2 + 1, float("nan")),
                              ("k", sk - 1, float("nan")), ("v", 5, float("nan")), ("v", sk - 1, float("inf"))):
@@ -99,9 +100,7 @@ def test_key_pieces_keep_nan_and_infinities(b, sq, sk, qh, kvh, causal):
         bad[name] = bad[name].clone()
         bad[name][0, row, 0, 77] = value
         out, lse = run_bshd(bad["q"], bad["k"], bad["v"], causal)
-        plain_out, plain_lse, cut = plain_workspace_forward(bad["q"], bad["k"], bad["v"], causal)
-        if torch.cuda.get_device_properties(0).multi_processor_count == 148:
-            assert cut
+        plain_out, plain_lse = plain_workspace_forward(bad["q"], bad["k"], bad["v"], causal)
         where = f"{name}[{row}] = {value}"
         assert not torch.isfinite(plain_out).all(), where
         assert torch.equal(torch.isnan(out), torch.isnan(plain_out)), where
