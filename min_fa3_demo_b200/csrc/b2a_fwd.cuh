@@ -47,6 +47,8 @@ constexpr int kTileM = 128;          // query rows per tile
 constexpr int kTileN = 128;          // key rows per K/V block
 constexpr int kFwdTilesPerCta = 2;   // tiles per work item
 constexpr int kFwdRowsPerWork = kTileM * kFwdTilesPerCta;
+constexpr int kFwdRowsPerWorkLog2 = 8;
+static_assert(kFwdRowsPerWork == 1 << kFwdRowsPerWorkLog2, "");
 constexpr int kFwdStages = 4;        // K/V ring stages
 constexpr int kFwdThreads = 384;
 constexpr int kFwdSlots = 4;         // decoded work items in flight between the load warp and its consumers
@@ -233,7 +235,7 @@ __device__ __forceinline__ FwdWork fwd_decode_work(const FwdParams& p, int w, in
     wk.head = w - entry * per_entry;
     wk.shift = p.pack_shift;
     if (p.pack_shift > 0) {
-        part = wk.head / p.heads_k;      // 0 for fixed-length calls
+        if (p.cu_seqlens_q != nullptr) part = wk.head / p.heads_k;
         wk.head_k = wk.head - part * p.heads_k;
         wk.head = wk.head_k << p.pack_shift;
         if (p.causal && p.cu_seqlens_q != nullptr) part = (1 << p.pack_shift) - 1 - part;   // longest first
@@ -253,8 +255,8 @@ __device__ __forceinline__ FwdWork fwd_decode_work(const FwdParams& p, int w, in
         wk.n_full = ring_full_chunks(p.causal, d.ring_size, d.ring_rank, e.y) * (d.half_len / kTileN);
         wk.lse_base = static_cast<long long>(wk.head) * p.lse_head_stride + wk.q_begin;
     } else if (p.cu_seqlens_q == nullptr) {
-        const int rows = kFwdRowsPerWork >> wk.shift;
-        int nmb = (p.seqlen_q + rows - 1) / rows;
+        const int rows_log2 = kFwdRowsPerWorkLog2 - wk.shift;
+        int nmb = (p.seqlen_q + (1 << rows_log2) - 1) >> rows_log2;
         int b = entry / nmb;
         int mi = entry - b * nmb;
         int mblk = p.causal ? (nmb - 1 - mi) : mi;
@@ -262,7 +264,7 @@ __device__ __forceinline__ FwdWork fwd_decode_work(const FwdParams& p, int w, in
         wk.q_len = p.seqlen_q;
         wk.k_begin = b * p.seqlen_k;
         wk.k_len = p.seqlen_k;
-        wk.m0 = mblk * rows;
+        wk.m0 = mblk << rows_log2;
         wk.lse_base = static_cast<long long>(b) * p.lse_batch_stride +
                       static_cast<long long>(wk.head) * p.lse_head_stride;
     } else {
@@ -561,10 +563,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 const uint32_t slot = it % kFwdSlots;
                 ok = mbar_wait(wctx, smem_u32(&sh.sched_empty[slot]), ((it / kFwdSlots) & 1u) ^ 1u, 1);
                 if (!ok) break;
-                FwdWork wk = fwd_decode_work<kMode == kFwdSplit>(p, __shfl_sync(0xFFFFFFFFu, ticket, 0), total_work);
-                while (wk.valid && (wk.m0 >= wk.q_len || (wk.pair && (wk.head & 1)))) {   // no query rows
-                    if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);
+                FwdWork wk;
+#pragma unroll 1
+                while (true) {
                     wk = fwd_decode_work<kMode == kFwdSplit>(p, __shfl_sync(0xFFFFFFFFu, ticket, 0), total_work);
+                    if (!wk.valid || (wk.m0 < wk.q_len && !(wk.pair && (wk.head & 1)))) break;
+                    if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);   // an item without query rows
                 }
                 if (lane == 0) {
                     sh.work[slot] = wk;
@@ -596,7 +600,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                                        ((kv_it / kFwdStages) & 1u) ^ 1u, 3);
                         if (!ok) break;
                         ++kv_it;
-                        int row = wk.k_begin + (wk.j0 + j) * kTileN;
+                        int row = wk.k_begin + (kMode == kFwdSplit ? wk.j0 + j : j) * kTileN;
                         if (p.ring_docs != nullptr) {
                             bool remote = false;
                             row = ring_kv_row(p, wk, j, &remote);
@@ -661,15 +665,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 tc_commit_w(smem_u32(&sh.s_full[x]));
                 if (j == 0) tc_commit_w(smem_u32(&sh.q_empty[x]));
             };
-            // First S of tile x in an item with n blocks for it, n_max for the longer tile (whose last block comes first).
-            auto start_tile = [&](int x, int n, int n_max, uint32_t stage) -> bool {
-                if (n == 0) return true;
-                if (!mbar_wait(wctx, smem_u32(&sh.q_full[x]), q_cnt[x] & 1u, 5)) return false;
-                ++q_cnt[x];
-                tc_fence_after_sync();
-                if (n == n_max) issue_s(x, n - 1, stage);
-                return true;
-            };
             // P V of block j of tile x.
             auto add_pv = [&](int x, int j, int n, uint32_t stage) -> bool {
                 PH_MARK(0);
@@ -688,7 +683,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             };
             // Block counts of the next work item; `valid` = 0 when there is none.
             uint32_t sched_it = 0;
-            auto next_item = [&](int (&n)[2], int& n_max, int& valid) -> bool {
+            auto next_item = [&](int (&n)[2], int& valid) -> bool {
                 const uint32_t slot = sched_it % kFwdSlots;
                 if (!mbar_wait(wctx, smem_u32(&sh.sched_full[slot]), (sched_it / kFwdSlots) & 1u, 4)) return false;
                 ++sched_it;
@@ -700,7 +695,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 n[1] = __shfl_sync(0xFFFFFFFFu, wk.nblk[1], 0);
                 if (lane == 0) mbar_arrive(smem_u32(&sh.sched_empty[slot]));
                 __syncwarp();
-                n_max = max(n[0], n[1]);
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
                     if (n[x] > 0) {
@@ -710,78 +704,63 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 }
                 return true;
             };
-            int nblk[2] = {0, 0}, n_max = 0, valid = 1;
-            bool started = false;    // the item's first S has been issued behind the previous item's last P V
-            while (ok) {
-                if (!started) {
-                    while (ok && valid && n_max == 0) ok = next_item(nblk, n_max, valid);
-                    if (!ok || !valid) break;
-                    const uint32_t stage = kv_it % kFwdStages;
-                    ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage]), (kv_it / kFwdStages) & 1u, 6);
-                    if (!ok) break;
-                    ++kv_it;
-                    ok = start_tile(0, nblk[0], n_max, stage) && start_tile(1, nblk[1], n_max, stage);
-                    tc_commit_w(smem_u32(&sh.kv_empty[stage]));
-                }
-                for (int j = n_max - 1; j > 0 && ok; --j) {
-                    const uint32_t stage_v = kv_it % kFwdStages;
+            // One pass per block: P V of block j, and S of the block behind it, which behind an item's last block is the
+            // first one of the next item.  What comes before the first item, and an item without keys, is a pass without
+            // P V.  Only the one item behind a last block is looked at: looking past items without keys there could mean
+            // waiting for softmax warps that wait for tile B below.  There is one copy of this code for first, middle and
+            // last blocks, because a short launch feels every copy's instruction cache misses: with three copies 16 x 1,024
+            // causal, 8 over 2 heads, took 61.9 us instead of 60.3, and 6 x 384 18.0 instead of 17.4.
+            int nblk[2] = {0, 0}, j = 0, valid = 1;
+            while (valid) {
+                const bool pv = nblk[0] > 0 || nblk[1] > 0;
+                uint32_t stage_v = 0;
+                if (pv) {
+                    stage_v = kv_it % kFwdStages;
                     ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_v]), (kv_it / kFwdStages) & 1u, 7);
                     if (!ok) break;
                     ++kv_it;
-                    const uint32_t stage_k = kv_it % kFwdStages;
+                }
+                const uint32_t stage_k = kv_it % kFwdStages;
+                const bool last = j == 0;
+                int n_s[2] = {nblk[0], nblk[1]}, j_s = j - 1;   // of the S to be issued; j_s = -1: there is none
 #pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        if (j < nblk[x]) {
-                            ok = add_pv(x, j, nblk[x], stage_v);
+                for (int x = 0; x < 2; ++x) {
+                    if (j < nblk[x]) {
+                        ok = add_pv(x, j, nblk[x], stage_v);
+                        if (!ok) break;
+                    }
+                    if (x == 1 && pv) tc_commit_w(smem_u32(&sh.kv_empty[stage_v]));
+                    if (x == 0) {
+                        if (last) {
+                            ok = next_item(n_s, valid);
                             if (!ok) break;
+                            j_s = max(n_s[0], n_s[1]) - 1;
                         }
-                        if (x == 1) tc_commit_w(smem_u32(&sh.kv_empty[stage_v]));
-                        if (x == 0) {
+                        if (j_s >= 0) {
                             ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_k]), (kv_it / kFwdStages) & 1u, 9);
                             if (!ok) break;
                             tc_fence_after_sync();
                         }
-                        PH_MARK(3);
-                        if (j - 1 < nblk[x]) issue_s(x, j - 1, stage_k);
-                        if (x == 1) tc_commit_w(smem_u32(&sh.kv_empty[stage_k]));
-                        __syncwarp();
-                        PH_MARK(4);
                     }
-                    ++kv_it;
-                }
-                if (!ok) break;
-                // Last block, with the next item's first S behind it.  Only the one item behind this: looking past items
-                // without keys here could mean waiting for softmax warps that wait for tile B below.
-                int nblk_next[2] = {0, 0}, n_max_next = 0;
-                const uint32_t stage_v = kv_it % kFwdStages;
-                ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_v]), (kv_it / kFwdStages) & 1u, 7);
-                if (!ok) break;
-                ++kv_it;
-                const uint32_t stage_k = kv_it % kFwdStages;
-                if (nblk[0] > 0) ok = add_pv(0, 0, nblk[0], stage_v);
-                ok = ok && next_item(nblk_next, n_max_next, valid);
-                if (!ok) break;
-                if (n_max_next > 0) {
-                    ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_k]), (kv_it / kFwdStages) & 1u, 9) &&
-                         start_tile(0, nblk_next[0], n_max_next, stage_k);
-                    if (!ok) break;
+                    PH_MARK(3);
+                    if (last && n_s[x] > 0) {
+                        ok = mbar_wait(wctx, smem_u32(&sh.q_full[x]), q_cnt[x] & 1u, 5);
+                        if (!ok) break;
+                        ++q_cnt[x];
+                        tc_fence_after_sync();
+                    }
+                    if (j_s >= 0) {
+                        if (j_s < n_s[x]) issue_s(x, j_s, stage_k);
+                        if (x == 1) tc_commit_w(smem_u32(&sh.kv_empty[stage_k]));
+                    }
                     __syncwarp();
+                    PH_MARK(4);
                 }
-                if (nblk[1] > 0) ok = add_pv(1, 0, nblk[1], stage_v);
                 if (!ok) break;
-                tc_commit_w(smem_u32(&sh.kv_empty[stage_v]));
-                if (n_max_next > 0) {
-                    ok = start_tile(1, nblk_next[1], n_max_next, stage_k);
-                    if (!ok) break;
-                    tc_commit_w(smem_u32(&sh.kv_empty[stage_k]));
-                    __syncwarp();
-                    ++kv_it;
-                }
-                nblk[0] = nblk_next[0];
-                nblk[1] = nblk_next[1];
-                n_max = n_max_next;
-                started = n_max > 0;
-                if (!valid) break;
+                if (j_s >= 0) ++kv_it;
+                nblk[0] = n_s[0];
+                nblk[1] = n_s[1];
+                j = max(j_s, 0);
             }
             // Each CTA submits its two totals once (reference: include/min_fa3_kernel.h:618-625).
             if (p.stats != nullptr && lane == 0 && tile_visits != 0) {
@@ -843,7 +822,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             if (p.causal) {
                 tile_min_limit = min(tile_min_limit, tile_row0 + 1 + wk.k_len - wk.q_len);
             }
-            const int n_full = wk.n_full - wk.j0;   // blocks are counted from the piece's first one
+            const int n_full = kMode == kFwdSplit ? wk.n_full - wk.j0 : wk.n_full;   // blocks are counted from the piece's first one
 
             float m_used = -INFINITY;   // running reference max (raw score units)
             float l = 0.f;              // running row sum relative to m_used
