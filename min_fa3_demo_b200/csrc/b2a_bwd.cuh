@@ -130,8 +130,6 @@ struct BwdWork {
     // Only in kernels that cut items:
     int t0, t1;        // steps [t0, t1) of the item's (query head, query tile) sequence
     int splits;        // pieces of the item (1: not cut, 0: a piece that the item does not need)
-    int split;         // which piece this is
-    int item;          // number of the item among those that may be cut
 };
 
 // Query tile of step t (within one head): document-local first row and whether it is the
@@ -152,15 +150,17 @@ __host__ __device__ __forceinline__ int bwd_padded_begin(int cu_begin, int doc) 
     return ((cu_begin + 127) / 128) * 128 + 256 * doc;
 }
 
+// kFixed: known to be a fixed-length call when compiling.
+template <bool kFixed>
 __device__ __forceinline__ BwdWork bwd_decode_item(const BwdParams& p, int w) {
     BwdWork wk;
     // Work order: key/value heads are taken `sg_heads` at a time ("supergroup", sized by the host
     // so that the dQ accumulator rows being added to stay within L2); inside a supergroup the
     // entries run in list order (most expensive first) with the head minor.  BSHD applies this
     // per batch element.
-    const int entries = p.cu_seqlens_q == nullptr ? p.num_entries_host : *p.num_entries_dev;
+    const int entries = kFixed || p.cu_seqlens_q == nullptr ? p.num_entries_host : *p.num_entries_dev;
     int per_batch = entries, b_idx = 0;
-    const bool bshd = p.cu_seqlens_q == nullptr && p.ring_docs == nullptr;
+    const bool bshd = kFixed || (p.cu_seqlens_q == nullptr && p.ring_docs == nullptr);
     if (bshd && p.batch_minor != 0) {
         // Deterministic mode: key block major, then batch element, then head.  A block waits for
         // the previous block of the same (batch element, head); spreading the running CTAs over
@@ -195,7 +195,7 @@ __device__ __forceinline__ BwdWork bwd_decode_item(const BwdParams& p, int w) {
     wk.diag_tile = 0;
     wk.owner = 0;
     wk.owner_block = 0;
-    if (p.ring_docs != nullptr) {
+    if (!kFixed && p.ring_docs != nullptr) {
         const int4 e = p.ring_work[entry];
         const RingDoc& d = p.ring_docs[e.x];
         const int g = d.ring_size, r = d.ring_rank, s = e.y, hf = e.z, blk = e.w;
@@ -236,7 +236,7 @@ __device__ __forceinline__ BwdWork bwd_decode_item(const BwdParams& p, int w) {
         return wk;
     }
     int nblk;
-    if (p.cu_seqlens_q == nullptr) {
+    if (kFixed || p.cu_seqlens_q == nullptr) {
         int nnb = (p.seqlen_k + kTileN - 1) / kTileN;
         int b = entry / nnb;
         int ni = entry - b * nnb;
@@ -273,21 +273,19 @@ __device__ __forceinline__ BwdWork bwd_decode_item(const BwdParams& p, int w) {
 template <bool kSplit>
 __device__ __forceinline__ BwdWork bwd_decode_work(const BwdParams& p, int w) {
     const bool cut = kSplit && w >= p.whole_items;
-    int item = 0, split = 0;
+    int split = 0;                       // which piece this is
     if (cut) {
         const int c = w - p.whole_items;
-        item = c / p.max_splits;
+        const int item = c / p.max_splits;
         split = c - item * p.max_splits;
         w = p.whole_items + item;
     }
-    BwdWork wk = bwd_decode_item(p, w);
+    BwdWork wk = bwd_decode_item<kSplit>(p, w);   // only fixed-length calls are cut
     if (!kSplit) return wk;
     const int steps = (wk.count0 + wk.count1) * (p.heads_q / p.heads_k);
     wk.t0 = 0;
     wk.t1 = steps;
     wk.splits = 1;
-    wk.split = split;
-    wk.item = item;
     if (cut) {
         wk.splits = min(p.max_splits, max(1, (steps + p.split_steps - 1) / p.split_steps));
         if (split >= wk.splits) {
@@ -493,9 +491,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     int total_work = (p.cu_seqlens_q == nullptr ? p.num_entries_host : *p.num_entries_dev) * p.heads_k;
     if (kSplit) total_work += (total_work - p.whole_items) * (p.max_splits - 1);
     const int group = p.heads_q / p.heads_k;
+    const bool ring_mode = !kSplit && p.ring_docs != nullptr;
 
     // Copy CTAs (ring mode) first pull the other ranks' K/V blocks into the local arena.
-    if (p.ring_docs != nullptr && static_cast<int>(blockIdx.x) >= p.num_comp && p.comm_task_count > 0) {
+    if (ring_mode && static_cast<int>(blockIdx.x) >= p.num_comp && p.comm_task_count > 0) {
         bwd_ring_copy_role(p, sh, wctx, warp, lane);
         __syncthreads();
     }
@@ -533,7 +532,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 ok = mbar_wait(wctx, smem_u32(&sh.kv_empty), (item_cnt & 1u) ^ 1u, 2);
                 if (!ok) break;
                 ++item_cnt;
-                if (p.ring_docs != nullptr && wk.owner != p.my_rank && p.comm_task_count > 0) {
+                if (ring_mode && wk.owner != p.my_rank && p.comm_task_count > 0) {
                     ok = flag_wait(wctx, p.kv_flags + wk.k_row / kTileN, 23);
                     if (!ok) break;
                     fence_proxy_async_all();
@@ -938,7 +937,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             const int per_head = wk.count0 + wk.count1;
             const int t0 = bwd_first_step<kSplit>(wk), t1 = bwd_end_step<kSplit>(wk, group);
             const int steps = t1 - t0;
-            const bool ring = p.ring_docs != nullptr;
             const int kv_row = wk.n0 + i_row;
             const bool kv_valid = kv_row < wk.k_len;
             const int shift = wk.k_len - wk.q_len;     // key c visible to query r iff c <= r + shift
@@ -951,9 +949,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 ++step_it;
                 // Query row of column 0, in the coordinates of the key rows (document-local, or
                 // chunk-local for the diagonal tile of a ring work item).
-                const int q0 = (ring ? q_local - (q_local >= wk.seg_len ? wk.seg_len : 0) : q_local) + wg * 64;
+                const int q0 = (ring_mode ? q_local - (q_local >= wk.seg_len ? wk.seg_len : 0) : q_local) + wg * 64;
                 // Columns c < c_min are hidden from this key row by the causal rule.
-                const int c_min = (ring ? diag : p.causal != 0) ? (kv_row - shift - q0) : 0;
+                const int c_min = (ring_mode ? diag : p.causal != 0) ? (kv_row - shift - q0) : 0;
                 const bool need_mask = !kv_valid || c_min > 0;
 
                 // LSE2 / D of this tile arrive with Q.
@@ -1079,10 +1077,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 tc_fence_after_sync();
             }
             const uint32_t acc_tmem = tmem_base + lane_base + (wg == 0 ? kColDV : kColDK);
-            if (kSplit && wk.splits > 1) {
+            if (kSplit && steps != per_head * group) {
                 // Every piece stores its fp32 sums; bwd_combine_kernel adds them up.
                 float4* part = p.split_part +
-                               ((static_cast<long long>(wk.item) * p.max_splits + wk.split) * 2 + wg) * (32 * kTileM) + i_row;
+                               (static_cast<long long>(w - p.whole_items) * 2 + wg) * (32 * kTileM) + i_row;
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
                     uint32_t v[32];
@@ -1108,7 +1106,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
 #pragma unroll
                     for (int i = 0; i < 32; ++i) v[i] = 0u;
                 }
-                if (ring) {
+                if (ring_mode) {
                     // Owner-directed accumulation: add this rank's partial dK / dV tile into the
                     // fp32 accumulator of the rank that owns the key block (possibly over NVLink).
                     float* acc = (wg == 0 ? p.dv_accum_peer[wk.owner] : p.dk_accum_peer[wk.owner]) +
@@ -1145,7 +1143,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
         PH_PRINT("compute", 7);
     }
 
-    if (p.ring_docs != nullptr) {
+    if (ring_mode) {
         __threadfence_system();   // this thread's peer adds are performed before the CTA reports
     }
     tc_fence_before_sync();
@@ -1154,7 +1152,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
-    if (p.ring_docs != nullptr && threadIdx.x == 0) {
+    if (ring_mode && threadIdx.x == 0) {
         // The last CTA of this rank tells every rank (itself included) that all of this rank's
         // dK / dV contributions have been added.
         const int done = atomicAdd(p.done_ctas, 1);
