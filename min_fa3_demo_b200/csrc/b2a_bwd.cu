@@ -97,6 +97,11 @@ struct BwdSplit {
 // that can cut spills a little, and its steps take 1 to 2 % longer.  Measured (us, whole backward, not cut / cut): 2 x
 // 1,024 causal, 16 over 4 heads: 100 / 80; 1 x 4,096 causal, 8 over 2: 376 / 195; 1 x 2,048, 8 over 1: 305 / 85; 2 x
 // 3,001, 32 heads, the last of eleven rounds cut, which this leaves alone: 820 / 830.
+// That formula picks the number of pieces, but it holds half a piece against an uncut causal call too, whose shortest items
+// come last and fill the gaps.  So the call is then handed out item by item both ways (HandOut, whose ratio was within
+// 5 % of the measured one for calls of over 150 us), and the cut has to promise a twentieth: 1 x 8,382 causal, 16 over 4
+// heads, is 752 us uncut and was 864 cut; 2 x 1,837, 64 over 8, 420 and 476; 4 x 486 rows of 4,834 keys, 14 over 2, 162 and
+// 186.
 // Items below kBwdMinCutSteps steps are never cut: little is gained (1 x 512 causal, 32 over 8 heads, 16 steps: 63 / 58),
 // and the last bits of short calls stay the same however a batch is divided into calls.
 constexpr int kBwdMinCutSteps = 24;
@@ -110,12 +115,13 @@ BwdSplit plan_bwd_split(const b2a_bwd_args& a, int ctas) {
     const int tiles = (a.seqlen_q + kTileM - 1) / kTileM;
     const long long n = static_cast<long long>(tiles) * group;   // steps of the longest item
     if (n < kBwdMinCutSteps || items >= 16ll * ctas) return s;
-    double mean = 0;
-    for (long long i = 0; i < nnb; ++i) {
+    auto steps_of = [&](long long i) {   // of an item with key block i
         const long long first_row = std::max<long long>(0, i * kTileN + a.seqlen_q - a.seqlen_k);
-        mean += static_cast<double>(tiles - (a.is_causal ? std::min<long long>(tiles, first_row / kTileM) : 0));
-    }
-    mean *= static_cast<double>(group) / static_cast<double>(nnb);
+        return group * static_cast<int>(tiles - (a.is_causal ? std::min<long long>(tiles, first_row / kTileM) : 0));
+    };
+    double mean = 0;
+    for (long long i = 0; i < nnb; ++i) mean += steps_of(i);
+    mean /= static_cast<double>(nnb);
     const bool even = mean > 0.8 * n;
     const long long whole = even ? items / ctas * ctas : 0;
     const double cut = static_cast<double>(items - whole);
@@ -135,6 +141,23 @@ BwdSplit plan_bwd_split(const b2a_bwd_args& a, int ctas) {
     s.whole_items = static_cast<int>(whole);
     s.steps = static_cast<int>((n + best - 1) / best);
     s.items = items - whole;
+    // The same two calls handed out item by item.
+    const double all = mean * items + 4.0 * items * best;
+    HandOut uncut(ctas, all, n + 3.0), pieced(ctas, all, n + 3.0);
+    long long left_whole = whole, parts_cut = 0;
+    for (int b = 0; b < a.batch; ++b) {
+        for (long long i = 0; i < nnb; ++i) {
+            const int steps = steps_of(i);
+            const long long first = std::min<long long>(left_whole, a.heads_k), rest = a.heads_k - first;
+            const int k = std::min(best, std::max(1, (steps + s.steps - 1) / s.steps));
+            uncut.add(steps + 1, a.heads_k);
+            pieced.add(steps + 1, first);
+            pieced.add((steps + k - 1) / k + 1 + (k > 1 ? 2 : 0), rest * k);
+            left_whole -= first;
+            if (k > 1) parts_cut += rest * k;
+        }
+    }
+    if (pieced.end() + 2.0 + parts_cut / 32.0 > 0.95 * uncut.end()) return BwdSplit{};
     return s.total() > (128u << 20) ? BwdSplit{} : s;   // the caller's thread keeps the scratch of its latest call
 }
 
@@ -248,7 +271,8 @@ int b2a_bwd(const b2a_bwd_args* a, void* cuda_stream) {
     DeviceInfo dev{};
     int rc = current_device_info(&dev);
     if (rc != B2A_OK) return rc;
-    BwdSplit split = plan_bwd_split(*a, dev.sm_count);
+    BwdSplit split;
+    if (a->workspace_bytes > lay.total) split = plan_bwd_split(*a, dev.sm_count);
     if (a->workspace_bytes < lay.total + split.total()) split = BwdSplit{};   // b2a_bwd_workspace_bytes is enough to run
     rc = configure_bwd_kernel(dev, split.max_splits > 1);
     if (rc != B2A_OK) return rc;

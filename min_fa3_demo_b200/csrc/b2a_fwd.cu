@@ -47,6 +47,9 @@ struct FwdSplit {
 // storing a piece, three for the launch that adds up, and the time that writing and reading the pieces takes (about
 // 4 TB/s: they stay in L2).  Where items differ a lot in length (a square causal call) the dynamic hand-out packs them,
 // and the bound is the mean load plus half a piece.  A cut has to promise a twentieth: the model knows no better.
+// That formula picks the number of pieces, but it holds half a piece against an uncut causal call too, whose shortest items
+// come last and fill the gaps.  So the call is then handed out item by item both ways (HandOut), and again the cut has
+// to promise a twentieth: 1 x 6,829 causal, 8 over 2 heads, is 116 us uncut and was 127 cut.
 // Measured (us, not cut / cut): 512 rows against 16,384 keys, 32 over 8 heads, two pieces: 221 / 132; 2 x 3,001 rows
 // without a mask, 32 heads, the last of six rounds cut: 287 / 277; one square causal call of 2 x 1,024, 16 over 4 heads,
 // which this leaves alone: 39 / 49.
@@ -63,12 +66,13 @@ FwdSplit plan_fwd_split(const b2a_fwd_args& a, int ctas) {
     const long long tile_rows = static_cast<long long>(a.seqlen_q) << shift;
     s.tiles = tile_rows > kTileM ? 2 : 1;
     s.rows = static_cast<int>(std::min<long long>(tile_rows, kTileM));
-    double mean = 0;   // blocks of an item
-    for (long long i = 0; i < pieces; ++i) {
+    auto blocks_of = [&](long long i) {   // that an item of piece i goes through
         const long long last = std::min<long long>((i + 1) * rows, a.seqlen_q);
         const long long limit = a.is_causal ? std::min<long long>(a.seqlen_k, last + a.seqlen_k - a.seqlen_q) : a.seqlen_k;
-        mean += limit <= 0 ? 0.0 : static_cast<double>((limit + kTileN - 1) / kTileN);
-    }
+        return limit <= 0 ? 0 : static_cast<int>((limit + kTileN - 1) / kTileN);
+    };
+    double mean = 0;   // blocks of an item
+    for (long long i = 0; i < pieces; ++i) mean += blocks_of(i);
     mean /= static_cast<double>(pieces);
     const bool even = mean > 0.8 * n;
     // Items of one length: only those of the last, incomplete round are cut.
@@ -91,6 +95,23 @@ FwdSplit plan_fwd_split(const b2a_fwd_args& a, int ctas) {
     s.max_splits = best;
     s.blocks = (n + best - 1) / best;
     s.items = items - whole;
+    // The same two calls handed out item by item.
+    const double steps = mean * items + 3.0 * items * best;
+    HandOut uncut(ctas, steps, n + 2), pieced(ctas, steps, n + 2);
+    long long left_whole = whole, parts_cut = 0;
+    for (int b = 0; b < a.batch; ++b) {
+        for (long long i = 0; i < pieces; ++i) {
+            const int blocks = blocks_of(a.is_causal ? pieces - 1 - i : i);
+            const long long first = std::min<long long>(left_whole, a.heads_k), rest = a.heads_k - first;
+            const int k = std::min(best, std::max(1, (blocks + s.blocks - 1) / s.blocks));
+            uncut.add(blocks + 1, a.heads_k);
+            pieced.add(blocks + 1, first);
+            pieced.add((blocks + k - 1) / k + 1 + (k > 1 ? 1 : 0), rest * k);
+            left_whole -= first;
+            if (k > 1) parts_cut += rest * k;
+        }
+    }
+    if (pieced.end() + 3.0 + parts_cut * piece_bytes / 6.8e6 > 0.95 * uncut.end()) return FwdSplit{};
     const size_t parts = static_cast<size_t>(cut) * best * s.tiles;
     s.stat_bytes = align_up(parts * s.rows * sizeof(float2), 256);
     s.o_bytes = align_up(parts * s.rows * kHeadDim * sizeof(float), 256);
@@ -278,7 +299,8 @@ int b2a_fwd(const b2a_fwd_args* a, void* cuda_stream) {
 
     auto* hdr = static_cast<WorkspaceHeader*>(a->workspace);
     int2* work_list = reinterpret_cast<int2*>(hdr + 1);
-    FwdSplit split = plan_fwd_split(*a, dev.sm_count);
+    FwdSplit split;
+    if (a->workspace_bytes > need) split = plan_fwd_split(*a, dev.sm_count);
     if (a->workspace_bytes < need + split.total()) split = FwdSplit{};   // b2a_fwd_workspace_bytes is enough to run
     uint8_t* split_ws = static_cast<uint8_t*>(a->workspace) + need;
     B2A_CUDA_OK(cudaMemsetAsync(hdr, 0, sizeof(WorkspaceHeader), stream));

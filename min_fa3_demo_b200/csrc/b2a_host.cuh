@@ -81,6 +81,35 @@ int noalloc_scratch_ptr(void** out);
 // Returns fn's code the first time and B2A_OK afterwards.
 int once_per_device(int device, int slot, int (*fn)());
 
+// How long a list of work items takes when each CTA takes the next item as soon as it is done with its last, in the unit of
+// the items' lengths (whole steps).  Times are kept as counts of CTAs per step, so an add() of equal items costs a few
+// instructions and the whole a microsecond or two.
+class HandOut {
+public:
+    // total, longest: at least the sum and the maximum of all lengths that will be added (they set the resolution).
+    HandOut(int ctas, double total, double longest) : unit_(1 + static_cast<int>((total / ctas + longest) / (kSlots / 2))) {
+        free_[0] = ctas;
+    }
+    void add(int length, long long times) {
+        const int d = (length + unit_ - 1) / unit_;
+        while (times > 0) {
+            while (free_[now_] == 0) ++now_;
+            const int n = static_cast<int>(times < free_[now_] ? times : free_[now_]);
+            const int end = now_ + d < kSlots ? now_ + d : kSlots - 1;
+            free_[now_] -= n;
+            free_[end] += n;
+            times -= n;
+            if (end > last_) last_ = end;
+        }
+    }
+    double end() const { return static_cast<double>(last_) * unit_; }
+
+private:
+    static constexpr int kSlots = 4096;
+    int unit_, now_ = 0, last_ = 0;
+    int free_[kSlots] = {};
+};
+
 // Raises the dynamic shared-memory limit of the forward kernel in a FwdMode once per device (b2a_fwd.cu).
 int configure_fwd_kernel(const DeviceInfo& dev, int mode);
 

@@ -12,7 +12,7 @@ import min_fa3_op
 from min_fa3_demo_b200 import _cabi
 from min_fa3_demo_b200 import min_fa3_op as min_fa3_op_impl
 from conftest import from_bf16_bits, load_golden
-from gpu_util import assert_lse, assert_within, bound, make_bshd, make_varlen, varlen_bf16_errors
+from gpu_util import assert_cut, assert_lse, assert_within, bound, make_bshd, make_varlen, varlen_bf16_errors
 from oracle import attention_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -84,6 +84,20 @@ def test_bshd_backward_cut_items(b, sq, sk, qh, kvh, causal, deterministic):
     torch.cuda.synchronize()
     for name, ours, ref in zip(("dq", "dk", "dv"), held[-3:], (rq, rk, rv)):
         assert_within(f"{name} (plain workspace)", ours, ref, e[name])
+
+
+@pytest.mark.parametrize("cut,b,sq,sk,qh,kvh,causal", [
+    (True, 2, 1024, 1024, 16, 4, True),      # 104 us uncut, 81 cut
+    (True, 1, 4096, 4096, 8, 2, True),       # 305 and 152
+    (True, 3, 3906, 3906, 24, 8, False),     # 1,699 and 1,464: the last, incomplete round
+    (False, 1, 512, 512, 32, 8, True),       # 16 steps
+    (False, 1, 8382, 8382, 16, 4, True),     # 752 and 864: the shortest items come last anyway
+    (False, 2, 1837, 1837, 64, 8, True),     # 420 and 476
+    (False, 4, 486, 4834, 14, 2, True),      # 162 and 186
+    (False, 3, 1920, 1920, 16, 4, True),     # 183 and 188
+])
+def test_which_calls_are_cut(cut, b, sq, sk, qh, kvh, causal):
+    assert_cut(cut, "bwd", b, sq, sk, qh, kvh, causal)
 
 
 @pytest.mark.parametrize("sq,sk", [(256, 512), (300, 200)])

@@ -87,7 +87,7 @@ def test_bshd_forward_packed_rows_and_key_pieces(b, sq, sk, qh, kvh, causal):
 @pytest.mark.parametrize("b,sq,sk,qh,kvh,causal", [
     (2, 1, 4001, 8, 2, True),         # eight pieces
     (1, 300, 4096, 4, 4, False),      # two tiles, the second with 44 rows
-    (1, 2048, 2048, 8, 2, True),      # items of one piece and pieces without a block for the first tile
+    (1, 8192, 8192, 2, 1, True),      # items of one piece and pieces without a block for the first tile
 ])
 def test_key_pieces_keep_nan_and_infinities(b, sq, sk, qh, kvh, causal):
     # A NaN or an infinity shows in the same places whether the keys are cut or not: one in a query row, in a key (none of
@@ -108,6 +108,20 @@ def test_key_pieces_keep_nan_and_infinities(b, sq, sk, qh, kvh, causal):
         assert torch.equal(torch.isneginf(out), torch.isneginf(plain_out)), where
         assert torch.equal(torch.isnan(lse), torch.isnan(plain_lse)), where
         assert torch.equal(torch.isneginf(lse), torch.isneginf(plain_lse)), where
+
+
+@pytest.mark.parametrize("cut,b,sq,sk,qh,kvh,causal", [
+    (True, 1, 512, 16384, 32, 8, True),      # 218 us uncut, 151 cut
+    (True, 2, 3001, 3001, 32, 32, False),    # 322 and 306: the last of six rounds
+    (True, 1, 1, 4096, 8, 1, True),
+    (False, 1, 1, 1024, 8, 1, True),         # eight blocks, and nothing gained
+    (False, 1, 6829, 6829, 8, 2, True),      # 116 and 127: the shortest items come last anyway
+    (False, 1, 6192, 6192, 8, 1, True),      # 93 and 100
+    (False, 2, 1024, 1024, 16, 4, True),     # 39 and 49
+    (False, 1, 512, 16384, 24, 8, True),     # groups that are no power of two are not cut
+])
+def test_which_calls_are_cut(cut, b, sq, sk, qh, kvh, causal):
+    assert_cut(cut, "fwd", b, sq, sk, qh, kvh, causal)
 
 
 @pytest.mark.parametrize("tag,causal", [("full", False), ("causal", True)])
