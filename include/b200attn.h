@@ -99,6 +99,14 @@ size_t b2a_fwd_scratch_bytes(const b2a_fwd_args* args);
 int b2a_fwd(const b2a_fwd_args* args, void* cuda_stream);
 
 /*
+ * b2a_fwd with the partial results of a cut call in a buffer of their own (16-byte aligned, NULL for none) instead of
+ * behind b2a_fwd_workspace_bytes in the workspace.  A cut call needs b2a_fwd_scratch_bytes - b2a_fwd_workspace_bytes
+ * there and is not cut with less.  The buffer may be reused in stream order after the call, while the workspace,
+ * whose status word b2a_check_status reads, is kept.
+ */
+int b2a_fwd_with_scratch(const b2a_fwd_args* args, void* scratch, size_t scratch_bytes, void* cuda_stream);
+
+/*
  * Forward for callers that must not allocate device memory.  No counterpart in the
  * reference (its bindings allocate outputs and scratch on every call, bindings.cpp:267-269).
  *
@@ -177,6 +185,9 @@ size_t b2a_bwd_scratch_bytes(const b2a_bwd_args* args);
  * accumulation and the cast back to bf16.
  */
 int b2a_bwd(const b2a_bwd_args* args, void* cuda_stream);
+
+/* b2a_bwd with the partial results of a cut call in a buffer of their own, see b2a_fwd_with_scratch. */
+int b2a_bwd_with_scratch(const b2a_bwd_args* args, void* scratch, size_t scratch_bytes, void* cuda_stream);
 
 /* ------------------------------------------------------------------------- */
 /* Peer memory (single node, NVLink)                                          */

@@ -166,11 +166,13 @@ SIGNATURES = {
     "b2a_fwd_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
     "b2a_fwd_scratch_bytes": (c_size_t, [POINTER(FwdArgs)]),
     "b2a_fwd": (c_int32, [POINTER(FwdArgs), c_void_p]),
+    "b2a_fwd_with_scratch": (c_int32, [POINTER(FwdArgs), c_void_p, c_size_t, c_void_p]),
     "b2a_fwd_noalloc": (c_int32, [POINTER(FwdArgs), c_void_p]),
     "b2a_fwd_noalloc_scratch_limit": (c_size_t, []),
     "b2a_bwd_scratch_bytes": (c_size_t, [POINTER(BwdArgs)]),
     "b2a_bwd_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32, c_int32, c_int32, c_int32]),
     "b2a_bwd": (c_int32, [POINTER(BwdArgs), c_void_p]),
+    "b2a_bwd_with_scratch": (c_int32, [POINTER(BwdArgs), c_void_p, c_size_t, c_void_p]),
     "b2a_ipc_export": (c_int32, [c_void_p, c_void_p, POINTER(ctypes.c_uint64)]),
     "b2a_ipc_import": (c_int32, [c_void_p, ctypes.c_uint64, POINTER(c_void_p)]),
     "b2a_ipc_close": (c_int32, [c_void_p, ctypes.c_uint64]),

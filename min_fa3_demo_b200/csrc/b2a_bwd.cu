@@ -158,7 +158,7 @@ BwdSplit plan_bwd_split(const b2a_bwd_args& a, int ctas) {
         }
     }
     if (pieced.end() + 2.0 + parts_cut / 32.0 > 0.95 * uncut.end()) return BwdSplit{};
-    return s.total() > (128u << 20) ? BwdSplit{} : s;   // the caller's thread keeps the scratch of its latest call
+    return s.total() > (128u << 20) ? BwdSplit{} : s;   // callers allocate it for every call
 }
 
 // Adds up the pieces of cut items, in the order of their steps, and writes dV and dK * scale.  One CTA per 32 key rows of
@@ -241,6 +241,15 @@ size_t b2a_bwd_scratch_bytes(const b2a_bwd_args* a) {
 
 int b2a_bwd(const b2a_bwd_args* a, void* cuda_stream) {
     using namespace b2a;
+    if (a == nullptr || a->workspace == nullptr) return b2a_bwd_with_scratch(a, nullptr, 0, cuda_stream);
+    const size_t need =
+        bwd_layout(a->batch, a->seqlen_q, a->total_q, a->total_k, a->heads_q, a->cu_seqlens_q != nullptr).total;
+    if (a->workspace_bytes <= need) return b2a_bwd_with_scratch(a, nullptr, 0, cuda_stream);
+    return b2a_bwd_with_scratch(a, static_cast<uint8_t*>(a->workspace) + need, a->workspace_bytes - need, cuda_stream);
+}
+
+int b2a_bwd_with_scratch(const b2a_bwd_args* a, void* scratch, size_t scratch_bytes, void* cuda_stream) {
+    using namespace b2a;
     B2A_REQUIRE(a != nullptr, "args must not be NULL");
     B2A_REQUIRE(a->dout && a->q && a->k && a->v && a->out && a->lse,
                 "dout, q, k, v, out and lse must not be NULL");
@@ -262,6 +271,7 @@ int b2a_bwd(const b2a_bwd_args* a, void* cuda_stream) {
     B2A_REQUIRE(a->grid_blocks >= 0, "grid_blocks must be >= 0, got %d", a->grid_blocks);
     B2A_REQUIRE(a->workspace != nullptr && (reinterpret_cast<uintptr_t>(a->workspace) & 0xFF) == 0,
                 "workspace must be a 256-byte aligned device pointer");
+    B2A_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 0xF) == 0, "scratch must be 16-byte aligned");
     const BwdLayout lay = bwd_layout(a->batch, a->seqlen_q, a->total_q, a->total_k, a->heads_q, varlen);
     if (a->workspace_bytes < lay.total) {
         return fail(B2A_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, need %zu",
@@ -272,8 +282,8 @@ int b2a_bwd(const b2a_bwd_args* a, void* cuda_stream) {
     int rc = current_device_info(&dev);
     if (rc != B2A_OK) return rc;
     BwdSplit split;
-    if (a->workspace_bytes > lay.total) split = plan_bwd_split(*a, dev.sm_count);
-    if (a->workspace_bytes < lay.total + split.total()) split = BwdSplit{};   // b2a_bwd_workspace_bytes is enough to run
+    if (scratch != nullptr && scratch_bytes > 0) split = plan_bwd_split(*a, dev.sm_count);
+    if (scratch_bytes < split.total()) split = BwdSplit{};   // b2a_bwd_workspace_bytes is enough to run
     rc = configure_bwd_kernel(dev, split.max_splits > 1);
     if (rc != B2A_OK) return rc;
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
@@ -378,7 +388,7 @@ int b2a_bwd(const b2a_bwd_args* a, void* cuda_stream) {
     p.max_splits = split.max_splits;
     p.whole_items = split.whole_items;
     p.split_steps = split.steps;
-    p.split_part = reinterpret_cast<float4*>(ws + lay.total);
+    p.split_part = static_cast<float4*>(scratch);
     int grid = a->grid_blocks > 0 ? a->grid_blocks : dev.sm_count;
     if (work_items < grid) grid = static_cast<int>(work_items);
     if (grid < 1) grid = 1;

@@ -115,7 +115,7 @@ FwdSplit plan_fwd_split(const b2a_fwd_args& a, int ctas) {
     const size_t parts = static_cast<size_t>(cut) * best * s.tiles;
     s.stat_bytes = align_up(parts * s.rows * sizeof(float2), 256);
     s.o_bytes = align_up(parts * s.rows * kHeadDim * sizeof(float), 256);
-    return s.total() > (128ull << 20) ? FwdSplit{} : s;   // the caller's thread keeps the scratch of its latest call
+    return s.total() > (128ull << 20) ? FwdSplit{} : s;   // callers allocate it for every call
 }
 
 // ---------------------------------------------------------------------------------------
@@ -247,6 +247,14 @@ size_t b2a_fwd_scratch_bytes(const b2a_fwd_args* a) {
 
 int b2a_fwd(const b2a_fwd_args* a, void* cuda_stream) {
     using namespace b2a;
+    if (a == nullptr || a->workspace == nullptr) return b2a_fwd_with_scratch(a, nullptr, 0, cuda_stream);
+    const size_t need = b2a_fwd_workspace_bytes(a->batch, a->total_q, a->cu_seqlens_q != nullptr ? 1 : 0);
+    if (a->workspace_bytes <= need) return b2a_fwd_with_scratch(a, nullptr, 0, cuda_stream);
+    return b2a_fwd_with_scratch(a, static_cast<uint8_t*>(a->workspace) + need, a->workspace_bytes - need, cuda_stream);
+}
+
+int b2a_fwd_with_scratch(const b2a_fwd_args* a, void* scratch, size_t scratch_bytes, void* cuda_stream) {
+    using namespace b2a;
     B2A_REQUIRE(a != nullptr, "args must not be NULL");
     B2A_REQUIRE(a->q && a->k && a->v && a->out && a->lse, "q, k, v, out and lse must not be NULL");
     B2A_REQUIRE(a->head_dim == kHeadDim, "head_dim must be 128, got %d", a->head_dim);
@@ -277,6 +285,7 @@ int b2a_fwd(const b2a_fwd_args* a, void* cuda_stream) {
     }
     B2A_REQUIRE(a->workspace != nullptr && (reinterpret_cast<uintptr_t>(a->workspace) & 0xF) == 0,
                 "workspace must be a 16-byte aligned device pointer");
+    B2A_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 0xF) == 0, "scratch must be 16-byte aligned");
     const size_t need = b2a_fwd_workspace_bytes(a->batch, a->total_q, varlen ? 1 : 0);
     if (a->workspace_bytes < need) {
         return fail(B2A_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, need %zu",
@@ -300,9 +309,9 @@ int b2a_fwd(const b2a_fwd_args* a, void* cuda_stream) {
     auto* hdr = static_cast<WorkspaceHeader*>(a->workspace);
     int2* work_list = reinterpret_cast<int2*>(hdr + 1);
     FwdSplit split;
-    if (a->workspace_bytes > need) split = plan_fwd_split(*a, dev.sm_count);
-    if (a->workspace_bytes < need + split.total()) split = FwdSplit{};   // b2a_fwd_workspace_bytes is enough to run
-    uint8_t* split_ws = static_cast<uint8_t*>(a->workspace) + need;
+    if (scratch != nullptr && scratch_bytes > 0) split = plan_fwd_split(*a, dev.sm_count);
+    if (scratch_bytes < split.total()) split = FwdSplit{};   // b2a_fwd_workspace_bytes is enough to run
+    uint8_t* split_ws = static_cast<uint8_t*>(scratch);
     B2A_CUDA_OK(cudaMemsetAsync(hdr, 0, sizeof(WorkspaceHeader), stream));
 
     FwdParams p{};

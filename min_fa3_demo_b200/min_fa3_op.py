@@ -175,6 +175,12 @@ def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
+def _workspaces(plain: int, full: int, device: torch.device):
+    """Workspace of a call, and what it needs for partial results when it is cut: a buffer of its own, because the
+    workspace outlives the call (see _remember_workspace) and the partial results may take 128 MiB."""
+    return _workspace(plain, device), _workspace(full - plain, device) if full > plain else None
+
+
 def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
@@ -206,13 +212,11 @@ def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads
         args.prefetch_bytes = dst_k.numel() * dst_k.element_size()
         args.prefetch_blocks = int(blocks)
     with torch.cuda.device(q.device):
-        if may_cut:
-            nbytes = lib.b2a_fwd_scratch_bytes(ctypes.byref(args))
-        else:
-            nbytes = lib.b2a_fwd_workspace_bytes(batch, total_q, 0 if cu_q is None else 1)
-        ws = _workspace(nbytes, q.device)
+        nbytes = lib.b2a_fwd_workspace_bytes(batch, total_q, 0 if cu_q is None else 1)
+        full = lib.b2a_fwd_scratch_bytes(ctypes.byref(args)) if may_cut and cu_q is None else nbytes
+        ws, scratch = _workspaces(nbytes, full, q.device)
         args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
-        _cabi.check(lib.b2a_fwd(ctypes.byref(args), _stream_ptr(q.device)))
+        _cabi.check(lib.b2a_fwd_with_scratch(ctypes.byref(args), _ptr(scratch), full - nbytes, _stream_ptr(q.device)))
     return ws
 
 
@@ -235,14 +239,11 @@ def _call_bwd(dout, q, k, v, out, lse, dq, dk, dv, *, cu_q, cu_k, batch, seqlen_
     args.grid_blocks = 0
     args.softmax_scale = 0.0
     with torch.cuda.device(q.device):
-        if may_cut:
-            nbytes = lib.b2a_bwd_scratch_bytes(ctypes.byref(args))
-        else:
-            nbytes = lib.b2a_bwd_workspace_bytes(batch, total_q, total_k, heads_q, heads_k,
-                                                 0 if cu_q is None else 1)
-        ws = _workspace(nbytes, q.device)
+        nbytes = lib.b2a_bwd_workspace_bytes(batch, total_q, total_k, heads_q, heads_k, 0 if cu_q is None else 1)
+        full = lib.b2a_bwd_scratch_bytes(ctypes.byref(args)) if may_cut and cu_q is None else nbytes
+        ws, scratch = _workspaces(nbytes, full, q.device)
         args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
-        _cabi.check(lib.b2a_bwd(ctypes.byref(args), _stream_ptr(q.device)))
+        _cabi.check(lib.b2a_bwd_with_scratch(ctypes.byref(args), _ptr(scratch), full - nbytes, _stream_ptr(q.device)))
     return ws
 
 

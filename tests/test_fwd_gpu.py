@@ -124,6 +124,24 @@ def test_which_calls_are_cut(cut, b, sq, sk, qh, kvh, causal):
     assert_cut(cut, "fwd", b, sq, sk, qh, kvh, causal)
 
 
+def test_partial_results_do_not_outlive_the_call():
+    # Kept for check_last_status is the workspace alone, not the 16 MiB and more of a cut call's partial results.
+    sizes = (1, 512, 8192, 32, 8, True)
+    assert_cut(True, "fwd", *sizes)
+    assert_cut(True, "bwd", 1, 2048, 2048, 32, 8, True)
+    q, k, v, _ = (t.cuda() for t in make_bshd(3, 1, 512, 32, 8, sk=8192))
+    q2, k2, v2, dout = (t.cuda() for t in make_bshd(4, 1, 2048, 32, 8))
+    out2, lse2 = min_fa3_op.forward(q2, k2, v2, True, return_lse=True)
+    min_fa3_op.forward(q, k, v, True)
+    min_fa3_op.backward(dout, q2, k2, v2, out2, lse2, True)
+    kept = min_fa3_op_impl._LAST.workspaces
+    lib = min_fa3_op_impl._cabi.load()
+    assert kept["forward"].numel() == lib.b2a_fwd_workspace_bytes(1, 512, 0)
+    assert kept["backward"].numel() == lib.b2a_bwd_workspace_bytes(1, 2048, 2048, 32, 8, 0)
+    min_fa3_op_impl.check_last_status("forward")
+    min_fa3_op_impl.check_last_status("backward")
+
+
 @pytest.mark.parametrize("tag,causal", [("full", False), ("causal", True)])
 def test_bshd_forward_golden(tag, causal):
     g = load_golden(f"bshd_{tag}")
