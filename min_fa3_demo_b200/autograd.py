@@ -79,12 +79,16 @@ def _looker_checks():
 
 
 _LOOKER_CHECKS = _looker_checks()
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
 
 
-def _plain_tensor(t: torch.Tensor) -> bool:
+def _plain_tensors(tensors) -> bool:
     # A lazily negated view's memory holds the values before the negation, and a zero tensor has no memory; the dispatcher
     # puts proper values in both before it calls a kernel.
-    return type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and not t.is_neg() and not t._is_zerotensor()
+    for t in tensors:
+        if type(t) not in _PLAIN_TYPES or not t.is_cuda or t.is_neg() or t._is_zerotensor():
+            return False
+    return True
 
 
 def _plain_call(*tensors: torch.Tensor) -> bool:
@@ -96,8 +100,8 @@ def _plain_call(*tensors: torch.Tensor) -> bool:
     return (not torch.compiler.is_compiling()
             and _LOOKER_CHECKS is not None
             and not torch.is_grad_enabled()
-            and all(map(_plain_tensor, tensors))
-            and not any(check() for check in _LOOKER_CHECKS))
+            and _plain_tensors(tensors)
+            and not any([check() for check in _LOOKER_CHECKS]))
 
 
 class _Attention(torch.autograd.Function):

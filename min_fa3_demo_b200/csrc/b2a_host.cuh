@@ -2,6 +2,7 @@
 // tensor-map construction, workspace layout.
 #pragma once
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -88,6 +89,9 @@ class HandOut {
 public:
     // total, longest: at least the sum and the maximum of all lengths that will be added (they set the resolution).
     HandOut(int ctas, double total, double longest) : unit_(1 + static_cast<int>((total / ctas + longest) / (kSlots / 2))) {
+        // Nothing starts later than the mean load, so times end at total / ctas + longest; half the room is spare.
+        slots_ = std::min(kSlots, 64 + 2 * static_cast<int>((total / ctas + longest) / unit_));
+        std::fill(free_, free_ + slots_, 0);
         free_[0] = ctas;
     }
     void add(int length, long long times) {
@@ -95,7 +99,7 @@ public:
         while (times > 0) {
             while (free_[now_] == 0) ++now_;
             const int n = static_cast<int>(times < free_[now_] ? times : free_[now_]);
-            const int end = now_ + d < kSlots ? now_ + d : kSlots - 1;
+            const int end = std::min(now_ + d, slots_ - 1);
             free_[now_] -= n;
             free_[end] += n;
             times -= n;
@@ -106,8 +110,8 @@ public:
 
 private:
     static constexpr int kSlots = 4096;
-    int unit_, now_ = 0, last_ = 0;
-    int free_[kSlots] = {};
+    int unit_, slots_, now_ = 0, last_ = 0;
+    int free_[kSlots];
 };
 
 // Raises the dynamic shared-memory limit of the forward kernel in a FwdMode once per device (b2a_fwd.cu).

@@ -165,8 +165,8 @@ def _check_device_capability(device: torch.device, what: str) -> None:
 # --------------------------------------------------------------------------------------
 # C-ABI plumbing
 # --------------------------------------------------------------------------------------
-def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream_ptr(device: torch.device) -> int:
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
@@ -175,10 +175,9 @@ def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
-def _workspaces(plain: int, full: int, device: torch.device):
-    """Workspace of a call, and what it needs for partial results when it is cut: a buffer of its own, because the
-    workspace outlives the call (see _remember_workspace) and the partial results may take 128 MiB."""
-    return _workspace(plain, device), _workspace(full - plain, device) if full > plain else None
+# Partial results of a cut call (up to 128 MiB) have a buffer of their own, because the workspace outlives the call (see
+# _remember_workspace).  Up to this size they may lie behind the workspace.
+_SCRATCH_KEPT = 65536
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -212,11 +211,20 @@ def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads
         args.prefetch_bytes = dst_k.numel() * dst_k.element_size()
         args.prefetch_blocks = int(blocks)
     with torch.cuda.device(q.device):
-        nbytes = lib.b2a_fwd_workspace_bytes(batch, total_q, 0 if cu_q is None else 1)
-        full = lib.b2a_fwd_scratch_bytes(ctypes.byref(args)) if may_cut and cu_q is None else nbytes
-        ws, scratch = _workspaces(nbytes, full, q.device)
+        ref = ctypes.byref(args)
+        nbytes = lib.b2a_fwd_scratch_bytes(ref) if may_cut else 0
+        scratch = None
+        if nbytes > _SCRATCH_KEPT or not may_cut:
+            plain = lib.b2a_fwd_workspace_bytes(batch, total_q, 0 if cu_q is None else 1)
+            if nbytes > plain:
+                scratch = _workspace(nbytes - plain, q.device)
+            nbytes = plain
+        ws = _workspace(nbytes, q.device)
         args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
-        _cabi.check(lib.b2a_fwd_with_scratch(ctypes.byref(args), _ptr(scratch), full - nbytes, _stream_ptr(q.device)))
+        if scratch is None:
+            _cabi.check(lib.b2a_fwd(ref, _stream_ptr(q.device)))
+        else:
+            _cabi.check(lib.b2a_fwd_with_scratch(ref, scratch.data_ptr(), scratch.numel(), _stream_ptr(q.device)))
     return ws
 
 
@@ -239,11 +247,16 @@ def _call_bwd(dout, q, k, v, out, lse, dq, dk, dv, *, cu_q, cu_k, batch, seqlen_
     args.grid_blocks = 0
     args.softmax_scale = 0.0
     with torch.cuda.device(q.device):
+        ref = ctypes.byref(args)
         nbytes = lib.b2a_bwd_workspace_bytes(batch, total_q, total_k, heads_q, heads_k, 0 if cu_q is None else 1)
-        full = lib.b2a_bwd_scratch_bytes(ctypes.byref(args)) if may_cut and cu_q is None else nbytes
-        ws, scratch = _workspaces(nbytes, full, q.device)
+        more = lib.b2a_bwd_scratch_bytes(ref) - nbytes if may_cut and cu_q is None else 0
+        ws = _workspace(nbytes, q.device)
         args.workspace, args.workspace_bytes = ws.data_ptr(), nbytes
-        _cabi.check(lib.b2a_bwd_with_scratch(ctypes.byref(args), _ptr(scratch), full - nbytes, _stream_ptr(q.device)))
+        if more == 0:
+            _cabi.check(lib.b2a_bwd(ref, _stream_ptr(q.device)))
+        else:
+            scratch = _workspace(more, q.device)
+            _cabi.check(lib.b2a_bwd_with_scratch(ref, scratch.data_ptr(), more, _stream_ptr(q.device)))
     return ws
 
 

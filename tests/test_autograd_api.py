@@ -36,7 +36,7 @@ def _stand_ins(monkeypatch):
     """Lets CPU tensors pass for CUDA ones, with cheap functions in the kernels' place; records direct calls."""
     direct = []
     monkeypatch.setattr(ag, "_require_cuda", lambda t, name: None)
-    monkeypatch.setattr(ag, "_plain_tensor", lambda t: type(t) in (torch.Tensor, torch.nn.Parameter))
+    monkeypatch.setattr(ag, "_plain_tensors", lambda tensors: all(type(t) in ag._PLAIN_TYPES for t in tensors))
     monkeypatch.setattr(ag._op, "forward", lambda q, k, v, causal, return_lse: (q * 2, q.new_zeros(
         (q.size(0), q.size(2), q.size(1)), dtype=torch.float32)))
     monkeypatch.setattr(ag._op, "backward", lambda dout, q, k, v, out, lse, causal, deterministic: (

@@ -47,15 +47,16 @@ def test_bshd_backward_vs_oracle(b, s, qh, kvh, causal):
 
 
 @pytest.mark.parametrize("deterministic", [False, True])
-@pytest.mark.parametrize("b,sq,sk,qh,kvh,causal", [
-    (1, 256, 256, 8, 2, True),        # too short to be cut
-    (1, 4000, 130, 2, 2, False),      # two key blocks, the second with two rows; 32 steps each
-    (1, 1000, 1000, 6, 2, True),      # groups of 3, 24 steps: the shortest that is cut
-    (1, 300, 1500, 32, 1, True),      # one group of all heads; most key blocks are seen by all query tiles
-    (1, 700, 300, 4, 1, True),        # query tiles that see no key
-    (1, 3100, 900, 20, 20, False),    # a full round of items and a rest, which alone is cut
+@pytest.mark.parametrize("b,sq,sk,qh,kvh,causal,cut", [
+    (1, 256, 256, 8, 2, True, False),       # too short to be cut
+    (1, 4000, 130, 2, 2, False, True),      # two key blocks, the second with two rows; 32 steps each
+    (1, 1000, 1000, 6, 2, True, True),      # groups of 3, 24 steps: the shortest that is cut
+    (1, 300, 1500, 32, 1, True, True),      # one group of all heads; most key blocks are seen by all query tiles
+    (1, 700, 300, 4, 1, True, True),        # query tiles that see no key
+    (1, 3100, 900, 20, 20, False, True),    # a full round of items and a rest, which alone is cut
 ])
-def test_bshd_backward_cut_items(b, sq, sk, qh, kvh, causal, deterministic):
+def test_bshd_backward_cut_items(b, sq, sk, qh, kvh, causal, cut, deterministic):
+    assert_cut(cut, "bwd", b, sq, sk, qh, kvh, causal)
     q, k, v, dout = make_bshd(17 + sq, b, sq, qh, kvh, sk=sk)
     out, lse, (dq, dk, dv) = fwd_bwd_bshd(q, k, v, dout, causal, deterministic=deterministic)
     min_fa3_op_impl.check_last_status("backward")

@@ -56,21 +56,25 @@ def test_bshd_forward_rectangular_causal(sq, sk):
 
 
 @pytest.mark.parametrize("causal", [False, True])
-@pytest.mark.parametrize("b,sq,sk,qh,kvh", [
-    (1, 1, 1024, 8, 1),       # one row of 8 heads: one tile, 8 of its rows used, keys cut into many pieces
-    (2, 1, 4001, 8, 2),       # ... with a ragged last key block
-    (1, 31, 2049, 16, 4),     # 124 packed rows
-    (1, 33, 3000, 16, 4),     # 132: four rows in the second tile
-    (1, 300, 4096, 4, 4),     # nothing to pack; the second item has 44 rows
-    (1, 200, 5000, 32, 1),    # 32 heads a row: four rows a tile
-    (1, 1030, 2048, 8, 2),    # causal: items of different lengths, cut into different numbers of pieces
-    (1, 100, 3000, 12, 2),    # groups of 6 are not packed and not cut: two heads an item
-    (1, 90, 1100, 6, 2),      # groups of 3
-    (1, 700, 1024, 256, 1),   # more heads than a tile has rows
-    (1, 9000, 70, 40, 40),    # causal: CTAs draw many items in a row that see no key
-    (1, 4500, 70, 24, 4),     # ... of two heads each
+@pytest.mark.parametrize("b,sq,sk,qh,kvh,cut", [
+    (1, 1, 1024, 8, 1, False),      # one row of 8 heads: one tile, 8 of its rows used
+    (1, 1, 4096, 8, 1, True),       # ... with the keys cut into eight pieces
+    (2, 1, 4001, 8, 2, True),       # ... with a ragged last key block
+    (5, 1, 4001, 32, 32, True),     # 160 items, of which the last 12 are cut
+    (1, 31, 2049, 16, 4, True),     # 124 packed rows
+    (1, 33, 3000, 16, 4, True),     # 132: four rows in the second tile
+    (1, 300, 4096, 4, 4, True),     # nothing to pack; the second item has 44 rows
+    (1, 200, 5000, 32, 1, True),    # 32 heads a row: four rows a tile
+    (1, 1030, 2048, 8, 2, True),    # causal: items of different lengths, cut into different numbers of pieces
+    (1, 2048, 2048, 4, 1, True),    # causal: items of one piece among them
+    (1, 100, 3000, 12, 2, False),   # groups of 6 are not packed and not cut: two heads an item
+    (1, 90, 1100, 6, 2, False),     # groups of 3
+    (1, 700, 1024, 256, 1, False),  # more heads than a tile has rows
+    (1, 9000, 70, 40, 40, False),   # causal: CTAs draw many items in a row that see no key
+    (1, 4500, 70, 24, 4, False),    # ... of two heads each
 ])
-def test_bshd_forward_packed_rows_and_key_pieces(b, sq, sk, qh, kvh, causal):
+def test_bshd_forward_packed_rows_and_key_pieces(b, sq, sk, qh, kvh, cut, causal):
+    assert_cut(cut, "fwd", b, sq, sk, qh, kvh, causal)
     q, k, v, _ = make_bshd(31 + sq, b, sq, qh, kvh, sk=sk)
     out, lse = run_bshd(q, k, v, causal)
     min_fa3_op_impl.check_last_status("forward")
@@ -122,6 +126,16 @@ def test_key_pieces_keep_nan_and_infinities(b, sq, sk, qh, kvh, causal):
 ])
 def test_which_calls_are_cut(cut, b, sq, sk, qh, kvh, causal):
     assert_cut(cut, "fwd", b, sq, sk, qh, kvh, causal)
+
+
+@pytest.mark.parametrize("blocks", [1, 7, 300])
+def test_a_cut_call_is_the_same_on_any_number_of_ctas(blocks):
+    sizes = (1, 300, 4096, 4, 4)
+    assert_cut(True, "fwd", *sizes, True)
+    q, k, v, _ = make_bshd(6, 1, 300, 4, 4, sk=4096)
+    out, lse = run_bshd(q, k, v, True)
+    out2, lse2 = run_bshd(q, k, v, True, manual_block_count=blocks)
+    assert torch.equal(out, out2) and torch.equal(lse, lse2)
 
 
 def test_partial_results_do_not_outlive_the_call():
