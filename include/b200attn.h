@@ -81,7 +81,10 @@ size_t b2a_fwd_workspace_bytes(int32_t batch, int32_t total_q, int32_t is_varlen
  * Scratch with which b2a_fwd is fastest for these arguments on the current device (pointers are not
  * looked at, except whether cu_seqlens_q is NULL).  Never less than b2a_fwd_workspace_bytes.  It is more
  * where a fixed-length call has too few query rows to keep every SM busy, e.g. a few tokens against long
- * K/V: with that much scratch the keys are cut as well and the partial results added up.
+ * K/V: with that much scratch the keys are cut as well and the partial results added up in fp32, in a fixed order.
+ * Whether and where a call is cut follows from its sizes and the device's SM count, not from grid_blocks, so the last
+ * bits of a sequence's results can depend on how many sequences and heads share the call.  A caller that wants them
+ * independent of that passes b2a_fwd_workspace_bytes: such a call is never cut.
  */
 size_t b2a_fwd_scratch_bytes(const b2a_fwd_args* args);
 
@@ -113,8 +116,8 @@ int b2a_fwd_with_scratch(const b2a_fwd_args* args, void* scratch, size_t scratch
  * Who needs it: code that runs where cudaMalloc is unavailable or forbidden -- a plugin
  * inside a serving runtime that hands out one fixed memory pool at start-up, a hard
  * real-time loop that may not touch the allocator, or a call site that owns q/k/v/out/lse
- * but has no way to size and pass a workspace.  Same computation and arguments as b2a_fwd,
- * except that args->workspace / workspace_bytes are ignored: the scratch (scheduler ticket,
+ * but has no way to size and pass a workspace.  Same computation and arguments as b2a_fwd
+ * with b2a_fwd_workspace_bytes (never cut), except that args->workspace / workspace_bytes are ignored: the scratch (scheduler ticket,
  * status word and the varlen work list) lives in a 64 KiB array built into the library,
  * resident on every GPU that loads it.  The call and everything under it use no cudaMalloc,
  * cudaFree or allocating library routine.

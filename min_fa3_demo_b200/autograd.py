@@ -17,7 +17,8 @@ module does the pairing once:
 
 The dense operators are registered with ``torch.library.custom_op`` (namespace ``b200attn``)
 with fake (meta) implementations, so they trace under ``torch.compile`` / fake tensors; there
-is no CPU implementation — calling them with CPU tensors raises.
+is no CPU implementation — calling them with CPU tensors raises.  Gradients are first order: those of
+``attention`` refuse to be differentiated again, those of the other two carry no graph.
 """
 
 from __future__ import annotations

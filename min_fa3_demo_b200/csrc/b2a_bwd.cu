@@ -94,9 +94,10 @@ struct BwdSplit {
 // the launch that adds up, and the time that writing and reading 128 KiB a piece takes (about 4 TB/s).  As in the
 // forward, items of one length run in rounds and only the last, incomplete one is cut; items that differ (causal) are
 // packed by the dynamic hand-out, which the mean load plus half a piece bounds.  A cut has to promise a tenth: the kernel
-// that can cut spills a little, and its steps take 1 to 2 % longer.  Measured (us, whole backward, not cut / cut): 2 x
-// 1,024 causal, 16 over 4 heads: 100 / 80; 1 x 4,096 causal, 8 over 2: 376 / 195; 1 x 2,048, 8 over 1: 305 / 85; 2 x
-// 3,001, 32 heads, the last of eleven rounds cut, which this leaves alone: 820 / 830.
+// that can cut spills a little, and its steps take about 1 % longer.  Measured (us, whole backward, not cut / cut): 2 x
+// 1,024 causal, 16 over 4 heads: 99 / 77; 1 x 4,096 causal, 8 over 2: 300 / 149; 1 x 2,048 causal, 8 over 1: 291 / 65; 3 x
+// 3,906 without a mask, 24 over 8, the last of six rounds: 1,746 / 1,480; 2 x 3,001 without a mask, 32 heads, the last of
+// eleven rounds cut, which this leaves alone: 820 / 830.
 // That formula picks the number of pieces, but it holds half a piece against an uncut causal call too, whose shortest items
 // come last and fill the gaps.  So the call is then handed out item by item both ways (HandOut, whose ratio was within
 // 5 % of the measured one for calls of over 150 us), and the cut has to promise a twentieth: 1 x 8,382 causal, 16 over 4

@@ -16,9 +16,9 @@
 // What bounds a tile is the chain softmax -> P V -> Q K^T (about 3,300 clk per block and tile against 2 x 1,024 of MMA for
 // the two tiles), so it does not stop between two work items: the first Q K^T of the next item is issued right behind the
 // last P V of the same tile, and the load warp hands out decoded work items through a ring of kFwdSlots, so that no other
-// warp waits for the ticket or for the document table.  With packed rows (fwd_pack_shift) that gives 5 % on 50 documents
-// of about 330 tokens (90.2 -> 85.9 us) and nothing measurable on long ones.  A warpgroup of its own for the epilogue was
-// slower: the softmax warps then have 176 registers instead of 216 and spill (1,750 -> 1,840 us on 4 x 8,192).
+// warp waits for the ticket or for the document table.  On 30 drawn packed batches that is worth 1 % (up to 4 % where
+// documents are short), and nothing measurable on long sequences.  A warpgroup of its own for the epilogue was slower: the
+// softmax warps then have 176 registers instead of 216 and spill (1,750 -> 1,840 us on 4 x 8,192).
 //
 // Tensor memory (512 columns): S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512).
 // P (bf16) overwrites the first 64 columns of its S tile and is consumed by the
@@ -629,7 +629,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 }
                 // The next ticket is taken no earlier than its K and V can be loaded: taken at the start of an item, a
                 // long one, it would tie the next to this CTA for as long (10 documents of up to 4,961 tokens without a
-                // mask: 190 us against 153).
+                // mask: 190 us against 157, with single passes from 154 to 179 as the last round falls, as it was without
+                // the ring).
                 if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);
             }
         } else if (warp == kFwdMmaWarp) {

@@ -303,7 +303,8 @@ def forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: bool, 
     """BSHD attention forward (reference: ``forward``, bindings.cpp:240-278).
 
     q ``[B, S, QH, 128]``, k/v ``[B, Sk, KVH, 128]`` bf16 contiguous; returns ``out`` like q and,
-    with ``return_lse``, the fp32 natural-log LSE ``[B, QH, S]``.
+    with ``return_lse``, the fp32 natural-log LSE ``[B, QH, S]``.  Repeated calls give the same bits;
+    the last bits can depend on how many sequences and heads share the call (``b2a_fwd_scratch_bytes``).
     """
     manual = _validate_manual_block_count(manual_block_count)
     _check_bshd(q, "q")
@@ -393,7 +394,9 @@ def backward(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
              ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """BSHD attention backward (reference: ``backward``, min_fa3_bwd_bindings.cu:156-253).
 
-    Returns ``(dq, dk, dv)``; caller-provided buffers are written in place and returned.
+    Returns ``(dq, dk, dv)``; caller-provided buffers are written in place and returned.  dk and dv
+    (and dq with ``deterministic``) repeat bit for bit; their last bits can depend on how many
+    sequences and heads share the call (``b2a_bwd_scratch_bytes``).
     """
     _check_bf16_cuda(q, "q", 4)
     _check_bf16_cuda(k, "k", 4)
