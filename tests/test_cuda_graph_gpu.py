@@ -8,7 +8,7 @@ import pytest
 import torch
 
 import min_fa3_op
-from gpu_util import make_bshd
+from gpu_util import assert_cut, make_bshd
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +46,29 @@ def test_forward_backward_capture_and_replay():
     dq_n, dk_n, dv_n = min_fa3_op.backward(dc, qc, kc, vc, out_n, lse_n, True, deterministic=True)
     torch.cuda.synchronize()
     assert torch.equal(out_g, out_n) and torch.equal(dq_g, dq_n) and torch.equal(dk_g, dk_n) and torch.equal(dv_g, dv_n)
+
+
+def test_cut_calls_capture_and_replay():
+    # The forward is cut along its keys, the backward along its steps; their partial results lie in the graph's pool, in
+    # buffers that are free again when each call has been captured.
+    assert_cut(True, "fwd", 1, 700, 6000, 8, 2, True)
+    assert_cut(True, "bwd", 1, 2000, 2000, 8, 2, True)
+    q, k, v, _ = (t.cuda() for t in make_bshd(57, 1, 700, 8, 2, sk=6000))
+    q2, k2, v2, dout = (t.cuda() for t in make_bshd(58, 1, 2000, 8, 2))
+
+    def run():
+        out, lse = min_fa3_op.forward(q, k, v, True, return_lse=True)
+        out2, lse2 = min_fa3_op.forward(q2, k2, v2, True, return_lse=True)
+        return (out, lse, out2, lse2, *min_fa3_op.backward(dout, q2, k2, v2, out2, lse2, True, deterministic=True))
+
+    eager = run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = run()
+    for _ in range(3):
+        for t in captured:
+            t.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(captured, eager))
