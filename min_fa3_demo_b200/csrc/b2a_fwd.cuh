@@ -9,21 +9,29 @@
 //
 //   warp  0-3   softmax warpgroup of tile A (one thread per query row)
 //   warp  4-7   softmax warpgroup of tile B
-//   warp  8     tcgen05.mma issue
+//   warp  8     Q K^T issue
 //   warp  9     TMA loads and work fetch
-//   warp 10-11  idle (10 stores in the copy roles)
+//   warp 10     P V issue (stores in the copy roles)
+//   warp 11     idle
 //
-// What bounds a tile is the chain softmax -> P V -> Q K^T (about 3,300 clk per block and tile against 2 x 1,024 of MMA for
-// the two tiles), so it does not stop between two work items: the first Q K^T of the next item is issued right behind the
-// last P V of the same tile, and the load warp hands out decoded work items through a ring of kFwdSlots, so that no other
-// warp waits for the ticket or for the document table.  On 30 drawn packed batches that is worth 1 % (up to 4 % where
-// documents are short), and nothing measurable on long sequences.  A warpgroup of its own for the epilogue was slower: the
-// softmax warps then have 176 registers instead of 216 and spill (1,750 -> 1,840 us on 4 x 8,192).
+// Tensor memory (512 columns): P_A [0,64) S [64,192) P_B [192,256) O_A [256,384) O_B [384,512).
+// A softmax warpgroup takes a whole row of S into registers, so the one S buffer serves both tiles in turn: while tile A
+// computes its probabilities, S of tile B is made, and the other way round.  P (bf16) has columns of its own and is consumed
+// by the P V MMA from tensor memory.  So neither Q K^T nor P V is on a tile's chain.  What bounds a pair of blocks is the
+// softmax of two warps per scheduler: about 2,650 clk against 2,048 of MMA (74 % of the tensor pipe; 3,200 and 62 % with S and
+// P of a tile in the same columns, where the chain was softmax -> P V -> Q K^T).  On long calls the clock gives a part of that
+// back (1.68 -> 1.59 GHz under the power cap): 8,192 keys, 32 over 8 heads: 852 -> 789 us, causal 454 -> 421; 4 x 2,048 causal
+// 152 -> 144; 512 rows against 16,384 keys 145 -> 132; one token for 16 x 4,001 60 -> 48.
+//   Q K^T and P V are issued by warps of their own: each instruction of an issuing warp waits its turn beside two dense
+// softmax warps, and one warp for both took 2,100 clk a tile and block for its waits and issues (8,192 causal: 516 us).
+// Leaving out the row maximum beyond an item's first block (the row sum tells when it is needed) was slower (443 against
+// 408 us): S then stays live through the exponentials.
 //
-// Tensor memory (512 columns): S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512).
-// P (bf16) overwrites the first 64 columns of its S tile and is consumed by the
-// P*V MMA straight from tensor memory.  K and V tiles travel through one shared
-// ring of 32 KiB stages in the order K(j0) V(j0) K(j0-1) V(j0-1) ...
+// Nothing stops between two work items: the load warp hands out decoded work items through a ring of kFwdSlots, and the next
+// item's first Q K^T only needs its Q and the S buffer.  A warpgroup of its own for the epilogue was slower: the softmax warps
+// then have 176 registers instead of 216 and spill (1,750 -> 1,840 us on 4 x 8,192).
+//
+// K and V tiles travel through two rings of 32 KiB stages, loaded in the order K(j) K(j-1) V(j) K(j-2) V(j-1) ...
 //
 // BSHD and varlen inputs share the code path: both are addressed as a flat
 // [tokens, heads, 128] tensor plus per-document (begin, length) pairs.
@@ -35,8 +43,8 @@ namespace b2a {
 
 // Which of the 16 four-element groups of a 64-column half row take two of their exponentials
 // from the FMA-pipe polynomial instead of the special-function unit (bit g: group g).
-// Measured in SM clocks per 128x128 block: none 1830, every second group (25 % of the
-// exponentials) 1797, all groups (50 %) 1866.
+// Measured, us on 8,192 keys, 32 over 8 heads, without a mask / causal: every fourth group (12.5 % of the exponentials)
+// 796 / 424, every second 789 / 421, three of four 802 / 428.
 #ifndef B2A_FWD_EXP_POLY_MASK
 #define B2A_FWD_EXP_POLY_MASK 0x5555u
 #endif
@@ -49,13 +57,16 @@ constexpr int kFwdTilesPerCta = 2;   // tiles per work item
 constexpr int kFwdRowsPerWork = kTileM * kFwdTilesPerCta;
 constexpr int kFwdRowsPerWorkLog2 = 8;
 static_assert(kFwdRowsPerWork == 1 << kFwdRowsPerWorkLog2, "");
-constexpr int kFwdStages = 4;        // K/V ring stages
+constexpr int kFwdStages = 2;        // stages of the K ring and of the V ring
 constexpr int kFwdThreads = 384;
 constexpr int kFwdSlots = 4;         // decoded work items in flight between the load warp and its consumers
-constexpr int kFwdMmaWarp = 8;
+constexpr int kFwdQkWarp = 8;        // issues Q K^T; owns tensor memory
+constexpr int kFwdPvWarp = 10;       // issues P V
 constexpr int kFwdLoadWarp = 9;
 constexpr int kFwdStoreWarp = 10;    // copy roles only
 constexpr int kFwdMaxSplits = 32;    // pieces of a key split
+// First tensor memory columns: P of the two tiles, the S that both use, O of the two tiles.
+constexpr uint32_t kFwdColP = 0, kFwdColPStep = 192, kFwdColS = 64, kFwdColO = 256;
 constexpr uint32_t kTileBytes = kTileM * kHeadDim * 2;   // 32 KiB bf16 tile
 constexpr uint32_t kHalfTileBytes = kTileBytes / 2;      // one 64-column half
 constexpr float kLog2e = 1.4426950408889634f;
@@ -178,15 +189,19 @@ __host__ __device__ __forceinline__ int fwd_items_per_entry(const FwdParams& p) 
 
 struct __align__(1024) FwdShared {
     uint8_t q[kFwdTilesPerCta][kTileBytes];
-    uint8_t kv[kFwdStages][kTileBytes];
+    uint8_t k[kFwdStages][kTileBytes];
+    uint8_t v[kFwdStages][kTileBytes];
     FwdWork work[kFwdSlots];
     uint64_t q_full[kFwdTilesPerCta];
     uint64_t q_empty[kFwdTilesPerCta];
-    uint64_t kv_full[kFwdStages];
-    uint64_t kv_empty[kFwdStages];
+    uint64_t k_full[kFwdStages];
+    uint64_t k_empty[kFwdStages];
+    uint64_t v_full[kFwdStages];
+    uint64_t v_empty[kFwdStages];
     uint64_t s_full[kFwdTilesPerCta];
+    uint64_t s_empty;
     uint64_t p_full[kFwdTilesPerCta];
-    uint64_t o_full[kFwdTilesPerCta];
+    uint64_t pv_done[kFwdTilesPerCta];
     uint64_t sched_full[kFwdSlots];
     uint64_t sched_empty[kFwdSlots];
     uint64_t comm_full[6];
@@ -499,15 +514,18 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             mbar_init(smem_u32(&sh.q_empty[i]), 1);
             mbar_init(smem_u32(&sh.s_full[i]), 1);
             mbar_init(smem_u32(&sh.p_full[i]), kTileM);
-            mbar_init(smem_u32(&sh.o_full[i]), 1);
+            mbar_init(smem_u32(&sh.pv_done[i]), 1);
         }
+        mbar_init(smem_u32(&sh.s_empty), kTileM);
         for (int i = 0; i < kFwdStages; ++i) {
-            mbar_init(smem_u32(&sh.kv_full[i]), 1);
-            mbar_init(smem_u32(&sh.kv_empty[i]), 1);
+            mbar_init(smem_u32(&sh.k_full[i]), 1);
+            mbar_init(smem_u32(&sh.k_empty[i]), 1);
+            mbar_init(smem_u32(&sh.v_full[i]), 1);
+            mbar_init(smem_u32(&sh.v_empty[i]), 1);
         }
         for (int i = 0; i < kFwdSlots; ++i) {
             mbar_init(smem_u32(&sh.sched_full[i]), 1);
-            mbar_init(smem_u32(&sh.sched_empty[i]), 1 + 2 * 4);  // MMA warp + 8 softmax warps
+            mbar_init(smem_u32(&sh.sched_empty[i]), 2 + 2 * 4);  // MMA warps + 8 softmax warps
         }
         for (int i = 0; i < 6; ++i) {
             mbar_init(smem_u32(&sh.comm_full[i]), 1);
@@ -517,7 +535,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
         fence_mbar_init();
         fence_proxy_async_smem();
     }
-    if (warp == kFwdMmaWarp) {
+    if (warp == kFwdQkWarp) {
         tmem_alloc(smem_u32(&sh.tmem_base), 512);
         tmem_relinquish();
         tc_fence_before_sync();
@@ -551,8 +569,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             int total_work =
                 (p.cu_seqlens_q == nullptr ? p.num_entries_host : *p.num_entries_dev) * fwd_items_per_entry(p);
             if (kMode == kFwdSplit) total_work += (total_work - p.whole_items) * (p.max_splits - 1);
-            uint32_t kv_it = 0;
-            uint32_t q_cnt[2] = {0, 0};
+            uint32_t k_it = 0, v_it = 0;
+            uint32_t q_par = 0;      // bit x: phase of tile x's Q buffer
             bool ok = true;
             // Ring mode: true once all copy CTAs are done, i.e. every remote block has landed.
             bool all_landed = p.ring_docs == nullptr || p.comm_task_count == 0;
@@ -575,200 +593,167 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                     mbar_arrive(smem_u32(&sh.sched_full[slot]));
                 }
                 if (!wk.valid) break;
-                const int n_max = max(wk.nblk[0], wk.nblk[1]);
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    if (wk.nblk[x] > 0) {
-                        ok = mbar_wait(wctx, smem_u32(&sh.q_empty[x]), (q_cnt[x] & 1u) ^ 1u, 2);
-                        if (!ok) break;
-                        ++q_cnt[x];
-                        if (lane == 0) {
-                            const uint32_t bar = smem_u32(&sh.q_full[x]);
-                            const uint32_t dst = smem_u32(&sh.q[x][0]);
-                            const int row = wk.q_begin + fwd_tile_row0(wk, x);
-                            mbar_arrive_expect_tx(bar, kTileBytes);
-                            tma_load_3d(dst, &map_q, bar, 0, fwd_tile_head(wk, x), row);
-                            tma_load_3d(dst + kHalfTileBytes, &map_q, bar, 64, fwd_tile_head(wk, x), row);
+                const int n0 = wk.nblk[0], n1 = wk.nblk[1];
+                const int n_max = max(n0, n1);
+                auto load_q = [&](int x) {
+                    if ((x == 0 ? n0 : n1) == 0) return;
+                    ok = mbar_wait(wctx, smem_u32(&sh.q_empty[x]), ((q_par >> x) & 1u) ^ 1u, 2);
+                    if (!ok) return;
+                    q_par ^= 1u << x;
+                    if (lane == 0) {
+                        const uint32_t bar = smem_u32(&sh.q_full[x]);
+                        const uint32_t dst = smem_u32(&sh.q[x][0]);
+                        const int row = wk.q_begin + fwd_tile_row0(wk, x);
+                        mbar_arrive_expect_tx(bar, kTileBytes);
+                        tma_load_3d(dst, &map_q, bar, 0, fwd_tile_head(wk, x), row);
+                        tma_load_3d(dst + kHalfTileBytes, &map_q, bar, 64, fwd_tile_head(wk, x), row);
+                    }
+                };
+                // K or V of block j into the next stage of its ring.
+                auto load_kv = [&](int j, bool is_k, uint32_t& count) {
+                    const uint32_t stage = count % kFwdStages;
+                    ok = mbar_wait(wctx, smem_u32(is_k ? &sh.k_empty[stage] : &sh.v_empty[stage]),
+                                   ((count / kFwdStages) & 1u) ^ 1u, 3);
+                    if (!ok) return;
+                    ++count;
+                    int row = wk.k_begin + (kMode == kFwdSplit ? wk.j0 + j : j) * kTileN;
+                    if (p.ring_docs != nullptr) {
+                        bool remote = false;
+                        row = ring_kv_row(p, wk, j, &remote);
+                        if (remote && is_k && !all_landed) {
+                            int landed;
+                            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(landed) : "l"(p.copy_done)
+                                         : "memory");
+                            if (landed >= copy_ctas) {
+                                all_landed = true;
+                            } else {
+                                ok = flag_wait(wctx, p.kv_flags + row / kTileN, 13);
+                                if (!ok) return;
+                            }
+                            fence_proxy_async_all();
                         }
                     }
+                    if (lane == 0) {
+                        const uint32_t bar = smem_u32(is_k ? &sh.k_full[stage] : &sh.v_full[stage]);
+                        const uint32_t dst = smem_u32(is_k ? &sh.k[stage][0] : &sh.v[stage][0]);
+                        const CUtensorMap* map = is_k ? &map_k : &map_v;
+                        mbar_arrive_expect_tx(bar, kTileBytes);
+                        tma_load_3d(dst, map, bar, 0, wk.head_k, row);
+                        tma_load_3d(dst + kHalfTileBytes, map, bar, 64, wk.head_k, row);
+                    }
+                };
+                // In the order in which they are needed: Q K^T is one to two blocks further than P V.
+                if (n_max > 0) {
+                    const int opener = n0 >= n1 ? 0 : 1;   // the tile that has the first block
+                    load_q(opener);
+                    if (ok) load_kv(n_max - 1, true, k_it);
+                    if (ok) load_q(opener ^ 1);
                 }
                 for (int j = n_max - 1; j >= 0 && ok; --j) {
-#pragma unroll
-                    for (int kv = 0; kv < 2; ++kv) {
-                        const uint32_t stage = kv_it % kFwdStages;
-                        ok = mbar_wait(wctx, smem_u32(&sh.kv_empty[stage]),
-                                       ((kv_it / kFwdStages) & 1u) ^ 1u, 3);
-                        if (!ok) break;
-                        ++kv_it;
-                        int row = wk.k_begin + (kMode == kFwdSplit ? wk.j0 + j : j) * kTileN;
-                        if (p.ring_docs != nullptr) {
-                            bool remote = false;
-                            row = ring_kv_row(p, wk, j, &remote);
-                            if (remote && kv == 0 && !all_landed) {
-                                int landed;
-                                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(landed) : "l"(p.copy_done)
-                                             : "memory");
-                                if (landed >= copy_ctas) {
-                                    all_landed = true;
-                                } else {
-                                    ok = flag_wait(wctx, p.kv_flags + row / kTileN, 13);
-                                    if (!ok) break;
-                                }
-                                fence_proxy_async_all();
-                            }
-                        }
-                        if (lane == 0) {
-                            const uint32_t bar = smem_u32(&sh.kv_full[stage]);
-                            const uint32_t dst = smem_u32(&sh.kv[stage][0]);
-                            const CUtensorMap* map = kv == 0 ? &map_k : &map_v;
-                            mbar_arrive_expect_tx(bar, kTileBytes);
-                            tma_load_3d(dst, map, bar, 0, wk.head_k, row);
-                            tma_load_3d(dst + kHalfTileBytes, map, bar, 64, wk.head_k, row);
-                        }
-                    }
+                    if (j > 0) load_kv(j - 1, true, k_it);
+                    if (ok) load_kv(j, false, v_it);
                 }
+                if (!ok) break;
                 // The next ticket is taken no earlier than its K and V can be loaded: taken at the start of an item, a
                 // long one, it would tie the next to this CTA for as long (10 documents of up to 4,961 tokens without a
                 // mask: 190 us against 157, with single passes from 154 to 179 as the last round falls, as it was without
                 // the ring).
                 if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);
             }
-        } else if (warp == kFwdMmaWarp) {
-            // ------------------------------------------------------------ MMA warp
+        } else if (warp == kFwdQkWarp || warp == kFwdPvWarp) {
+            // ------------------------------------------------------------ MMA warps
+            // Both go through the same (block, tile) pairs in the same order, each with no waits but its own.
+            const bool qk = warp == kFwdQkWarp;
             constexpr uint32_t idesc_qk = make_idesc_bf16(kTileM, kTileN, 0, 0);
             constexpr uint32_t idesc_pv = make_idesc_bf16(kTileM, kHeadDim, 0, 1);
-            uint32_t kv_it = 0;
-            uint32_t q_cnt[2] = {0, 0};
-            uint32_t p_cnt[2] = {0, 0};
             bool ok = true;
             unsigned int tile_visits = 0, kv_tile_reads = 0;   // CTA-local totals for p.stats
-            PH_DECL(8)   // 0 other, 1 wait p_full, 2 issue PV, 3 wait K, 4 issue S
-            const uint32_t s_tmem[2] = {tmem_base + 0u, tmem_base + 128u};
-            const uint32_t o_tmem[2] = {tmem_base + 256u, tmem_base + 384u};
-
-            // Descriptor low words of the Q tiles and of K/V stage 0 (a stage is 32 KiB further).
-            const uint32_t q_lo[2] = {desc_lo_kmajor(smem_u32(&sh.q[0][0])), desc_lo_kmajor(smem_u32(&sh.q[1][0]))};
-            const uint32_t k_lo0 = desc_lo_kmajor(smem_u32(&sh.kv[0][0]));
-            const uint32_t v_lo0 = desc_lo_mnmajor(smem_u32(&sh.kv[0][0]));
+            PH_DECL(8)   // 0 other, 1 wait K (and Q) / V, 2 wait S / P, 3 issue
+            // Descriptor low words of tile 0 / stage 0 (the next one is 32 KiB further).
+            const uint32_t q_lo0 = desc_lo_kmajor(smem_u32(&sh.q[0][0]));
+            const uint32_t k_lo0 = desc_lo_kmajor(smem_u32(&sh.k[0][0]));
+            const uint32_t v_lo0 = desc_lo_mnmajor(smem_u32(&sh.v[0][0]));
             constexpr uint32_t kStageStep = kTileBytes >> 4;
-
-            // S_x = Q_x * K^T for the K tile in `stage` (8 k-steps of 16 over head_dim).
-            auto issue_qk = [&](int x, uint32_t stage) {
-                umma_ss_kk_x8_w(s_tmem[x], q_lo[x], k_lo0 + stage * kStageStep, idesc_qk, 0u);
-            };
-            // O_x (+)= P_x * V for the V tile in `stage` (8 k-steps of 16 over keys).
-            auto issue_pv = [&](int x, uint32_t stage, uint32_t accumulate) {
-                umma_ts_x8_w(o_tmem[x], s_tmem[x], v_lo0 + stage * kStageStep, idesc_pv, accumulate);
-            };
-
-            auto issue_s = [&](int x, int j, uint32_t stage) {
-                issue_qk(x, stage);
-                tc_commit_w(smem_u32(&sh.s_full[x]));
-                if (j == 0) tc_commit_w(smem_u32(&sh.q_empty[x]));
-            };
-            // P V of block j of tile x.
-            auto add_pv = [&](int x, int j, int n, uint32_t stage) -> bool {
-                PH_MARK(0);
-                if (!mbar_wait(wctx, smem_u32(&sh.p_full[x]), p_cnt[x] & 1u, 8)) return false;
-                ++p_cnt[x];
-                tc_fence_after_sync();
-                PH_MARK(1);
-                issue_pv(x, stage, j != n - 1 ? 1u : 0u);
-                if (j == 0) tc_commit_w(smem_u32(&sh.o_full[x]));
-                __syncwarp();
-                PH_MARK(2);
-#ifdef B2A_PHASES
-                ph_[9] += 1;
-#endif
-                return true;
-            };
-            // Block counts of the next work item; `valid` = 0 when there is none.
-            uint32_t sched_it = 0;
-            auto next_item = [&](int (&n)[2], int& valid) -> bool {
-                const uint32_t slot = sched_it % kFwdSlots;
-                if (!mbar_wait(wctx, smem_u32(&sh.sched_full[slot]), (sched_it / kFwdSlots) & 1u, 4)) return false;
-                ++sched_it;
+            uint32_t kv_it = 0;   // K (V) blocks so far
+            uint32_t s_it = 0;    // S tiles so far
+            uint32_t par = 0;     // bit x: phase of tile x's Q (P)
+            for (uint32_t it = 0; ok; ++it) {
+                const uint32_t slot = it % kFwdSlots;
+                ok = mbar_wait(wctx, smem_u32(&sh.sched_full[slot]), (it / kFwdSlots) & 1u, 4);
+                if (!ok) break;
                 // Broadcast from lane 0 so that everything derived from the counts (ring stages,
                 // operand descriptors) is provably warp-uniform for the compiler.
                 const volatile FwdWork& wk = sh.work[slot];
-                valid = __shfl_sync(0xFFFFFFFFu, wk.valid, 0);
-                n[0] = __shfl_sync(0xFFFFFFFFu, wk.nblk[0], 0);
-                n[1] = __shfl_sync(0xFFFFFFFFu, wk.nblk[1], 0);
+                const int valid = __shfl_sync(0xFFFFFFFFu, wk.valid, 0);
+                const int nblk[2] = {__shfl_sync(0xFFFFFFFFu, wk.nblk[0], 0), __shfl_sync(0xFFFFFFFFu, wk.nblk[1], 0)};
                 if (lane == 0) mbar_arrive(smem_u32(&sh.sched_empty[slot]));
                 __syncwarp();
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    if (n[x] > 0) {
-                        tile_visits += 1;
-                        kv_tile_reads += static_cast<unsigned int>(n[x]);
-                    }
-                }
-                return true;
-            };
-            // One pass per block: P V of block j, and S of the block behind it, which behind an item's last block is the
-            // first one of the next item.  What comes before the first item, and an item without keys, is a pass without
-            // P V.  Only the one item behind a last block is looked at: looking past items without keys there could mean
-            // waiting for softmax warps that wait for tile B below.  There is one copy of this code for first, middle and
-            // last blocks, because a short launch feels every copy's instruction cache misses: with three copies 16 x 1,024
-            // causal, 8 over 2 heads, took 61.9 us instead of 60.3, and 6 x 384 18.0 instead of 17.4.
-            int nblk[2] = {0, 0}, j = 0, valid = 1;
-            while (valid) {
-                const bool pv = nblk[0] > 0 || nblk[1] > 0;
-                uint32_t stage_v = 0;
-                if (pv) {
-                    stage_v = kv_it % kFwdStages;
-                    ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_v]), (kv_it / kFwdStages) & 1u, 7);
-                    if (!ok) break;
-                    ++kv_it;
-                }
-                const uint32_t stage_k = kv_it % kFwdStages;
-                const bool last = j == 0;
-                int n_s[2] = {nblk[0], nblk[1]}, j_s = j - 1;   // of the S to be issued; j_s = -1: there is none
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    if (j < nblk[x]) {
-                        ok = add_pv(x, j, nblk[x], stage_v);
+                if (!valid) break;
+                tile_visits += (nblk[0] > 0) + (nblk[1] > 0);
+                kv_tile_reads += static_cast<unsigned int>(nblk[0] + nblk[1]);
+                if (qk) {
+                    for (int j = max(nblk[0], nblk[1]) - 1; j >= 0 && ok; --j) {
+                        const uint32_t stage = kv_it % kFwdStages;
+                        PH_MARK(0);
+                        ok = mbar_wait(wctx, smem_u32(&sh.k_full[stage]), (kv_it / kFwdStages) & 1u, 9);
                         if (!ok) break;
-                    }
-                    if (x == 1 && pv) tc_commit_w(smem_u32(&sh.kv_empty[stage_v]));
-                    if (x == 0) {
-                        if (last) {
-                            ok = next_item(n_s, valid);
+                        ++kv_it;
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            if (j >= nblk[x]) continue;
+                            if (j == nblk[x] - 1) {
+                                ok = mbar_wait(wctx, smem_u32(&sh.q_full[x]), (par >> x) & 1u, 5);
+                                if (!ok) break;
+                                par ^= 1u << x;
+                            }
+                            PH_MARK(1);
+                            // The softmax warps have taken the S before this one out of tensor memory.
+                            ok = mbar_wait(wctx, smem_u32(&sh.s_empty), (s_it & 1u) ^ 1u, 6);
                             if (!ok) break;
-                            j_s = max(n_s[0], n_s[1]) - 1;
-                        }
-                        if (j_s >= 0) {
-                            ok = mbar_wait(wctx, smem_u32(&sh.kv_full[stage_k]), (kv_it / kFwdStages) & 1u, 9);
-                            if (!ok) break;
+                            ++s_it;
+                            PH_MARK(2);
                             tc_fence_after_sync();
+                            umma_ss_kk_x8_w(tmem_base + kFwdColS, q_lo0 + x * kStageStep, k_lo0 + stage * kStageStep,
+                                            idesc_qk, 0u);
+                            tc_commit_w(smem_u32(&sh.s_full[x]));
+                            if (j == 0) tc_commit_w(smem_u32(&sh.q_empty[x]));
+                            __syncwarp();
+                            PH_MARK(3);
                         }
+                        tc_commit_w(smem_u32(&sh.k_empty[stage]));
                     }
-                    PH_MARK(3);
-                    if (last && n_s[x] > 0) {
-                        ok = mbar_wait(wctx, smem_u32(&sh.q_full[x]), q_cnt[x] & 1u, 5);
+                } else {
+                    for (int j = max(nblk[0], nblk[1]) - 1; j >= 0 && ok; --j) {
+                        const uint32_t stage = kv_it % kFwdStages;
+                        PH_MARK(0);
+                        ok = mbar_wait(wctx, smem_u32(&sh.v_full[stage]), (kv_it / kFwdStages) & 1u, 7);
                         if (!ok) break;
-                        ++q_cnt[x];
-                        tc_fence_after_sync();
+                        ++kv_it;
+                        PH_MARK(1);
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            if (j >= nblk[x]) continue;
+                            ok = mbar_wait(wctx, smem_u32(&sh.p_full[x]), (par >> x) & 1u, 8);
+                            if (!ok) break;
+                            par ^= 1u << x;
+                            PH_MARK(2);
+                            tc_fence_after_sync();
+                            umma_ts_x8_w(tmem_base + kFwdColO + x * 128u, tmem_base + kFwdColP + x * kFwdColPStep,
+                                         v_lo0 + stage * kStageStep, idesc_pv, j != nblk[x] - 1 ? 1u : 0u);
+                            tc_commit_w(smem_u32(&sh.pv_done[x]));
+                            __syncwarp();
+                            PH_MARK(3);
+                        }
+                        tc_commit_w(smem_u32(&sh.v_empty[stage]));
                     }
-                    if (j_s >= 0) {
-                        if (j_s < n_s[x]) issue_s(x, j_s, stage_k);
-                        if (x == 1) tc_commit_w(smem_u32(&sh.kv_empty[stage_k]));
-                    }
-                    __syncwarp();
-                    PH_MARK(4);
                 }
-                if (!ok) break;
-                if (j_s >= 0) ++kv_it;
-                nblk[0] = n_s[0];
-                nblk[1] = n_s[1];
-                j = max(j_s, 0);
             }
             // Each CTA submits its two totals once (reference: include/min_fa3_kernel.h:618-625).
-            if (p.stats != nullptr && lane == 0 && tile_visits != 0) {
+            if (qk && p.stats != nullptr && lane == 0 && tile_visits != 0) {
                 atomicAdd(p.stats, static_cast<unsigned long long>(tile_visits));
                 atomicAdd(p.stats + 1, static_cast<unsigned long long>(kv_tile_reads));
             }
-            PH_PRINT("fwd mma", 5);
+            PH_PRINT("fwd mma", 4);
         }
     } else {
         // ---------------------------------------------------------------- softmax warpgroups
@@ -776,10 +761,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
         const int x = warp >> 2;                        // tile index
         const int r = (warp & 3) * 32 + lane;           // row within the tile
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t s_tmem = tmem_base + lane_base + static_cast<uint32_t>(x) * 128u;
-        const uint32_t o_tmem = tmem_base + lane_base + 256u + static_cast<uint32_t>(x) * 128u;
+        const uint32_t s_tmem = tmem_base + lane_base + kFwdColS;
+        const uint32_t p_tmem = tmem_base + lane_base + kFwdColP + static_cast<uint32_t>(x) * kFwdColPStep;
+        const uint32_t o_tmem = tmem_base + lane_base + kFwdColO + static_cast<uint32_t>(x) * 128u;
         uint32_t s_cnt = 0;
-        uint32_t o_cnt = 0;
+        uint32_t pv_cnt = 0;
         bool ok = true;
         const float sl2 = p.scale_log2;
         PH_DECL(8)   // 0 other, 1 wait s_full, 2 tmem load, 3 max/rescale, 4 exp + store, 5 st wait + arrive
@@ -810,9 +796,18 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                     ok = mbar_wait(wctx, smem_u32(&sh.s_full[x]), s_cnt & 1u, 11);
                     if (!ok) break;
                     ++s_cnt;
+                    mbar_arrive(smem_u32(&sh.s_empty));
+                    if (j != nblk - 1) {   // no P of this block before the other warps' P of the last one is consumed
+                        ok = mbar_wait(wctx, smem_u32(&sh.pv_done[x]), pv_cnt & 1u, 12);
+                        if (!ok) break;
+                        ++pv_cnt;
+                    }
                     mbar_arrive(smem_u32(&sh.p_full[x]));
                 }
-                if (nblk > 0) ++o_cnt;
+                if (nblk > 0) {
+                    ok = ok && mbar_wait(wctx, smem_u32(&sh.pv_done[x]), pv_cnt & 1u, 12);
+                    ++pv_cnt;
+                }
                 release();
                 continue;
             }
@@ -848,36 +843,47 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                     for (int i = 0; i < 32; ++i) s[c * 32 + i] = __uint_as_float(t[i]);
                 }
                 tmem_wait_ld();
+                tc_fence_before_sync();
+                mbar_arrive(smem_u32(&sh.s_empty));
                 PH_MARK(2);
 
                 const int n0 = (j - n_full) * kTileN;   // own-chunk column of the block
                 if (j >= n_full && n0 + kTileN > tile_min_limit) {
+                    // One bit per visible column of 32: half the instructions of 128 comparisons.
                     const int lim = col_limit - n0;
 #pragma unroll
-                    for (int i = 0; i < kTileN; ++i) {
-                        if (i >= lim) s[i] = -INFINITY;
+                    for (int c = 0; c < 4; ++c) {
+                        const int vis = min(max(lim - c * 32, 0), 32);
+                        const uint32_t bits = vis == 32 ? 0xFFFFFFFFu : (1u << vis) - 1u;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            if (!((bits >> i) & 1u)) s[c * 32 + i] = -INFINITY;
+                        }
                     }
                 }
 
-                // Row maximum with four independent chains of 3-input maxima (a single chain of
-                // 127 dependent operations would be pure latency for the one warp per scheduler).
+                // Row maximum with eight independent chains: a single one would be pure latency, and 3-input maxima
+                // run at half the rate (2.0 clk a warp against 1.05, so the same time) with longer chains.
                 float bm;
                 {
-                    float m0 = s[0], m1 = s[1], m2 = s[2], m3 = s[3];
+                    float m[8];
 #pragma unroll
-                    for (int i = 4; i + 7 < kTileN; i += 8) {
-                        m0 = max3(m0, s[i], s[i + 1]);
-                        m1 = max3(m1, s[i + 2], s[i + 3]);
-                        m2 = max3(m2, s[i + 4], s[i + 5]);
-                        m3 = max3(m3, s[i + 6], s[i + 7]);
-                    }
-                    // 4 + 15 * 8 = 124 consumed; four left
-                    m0 = max3(m0, s[124], s[125]);
-                    m1 = max3(m1, s[126], s[127]);
-                    bm = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+                    for (int i = 0; i < 8; ++i) m[i] = s[i];
+#pragma unroll
+                    for (int i = 8; i < kTileN; ++i) m[i & 7] = fmaxf(m[i & 7], s[i]);
+                    bm = fmaxf(max3(max3(m[0], m[1], m[2]), m[3], m[4]), max3(m[5], m[6], m[7]));
                 }
 
+                // The P V of the tile's previous block must be done before O is rescaled and before P is overwritten.
                 const bool first = (j == nblk - 1);
+                bool pv_pending = !first;
+                auto wait_pv = [&]() -> bool {
+                    if (!mbar_wait(wctx, smem_u32(&sh.pv_done[x]), pv_cnt & 1u, 12)) return false;
+                    ++pv_cnt;
+                    tc_fence_after_sync();
+                    pv_pending = false;
+                    return true;
+                };
                 const float m_new = fmaxf(m_used, bm);
                 if (first) {
                     m_used = m_new;
@@ -888,7 +894,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                             (m_new == -INFINITY) ? 1.f : fast_exp2((m_used - m_new) * sl2);
                         l *= factor;
                         m_used = m_new;
-#pragma unroll
+                        ok = wait_pv();
+                        if (!ok) break;
+#pragma unroll 1   // rare
                         for (int c = 0; c < 4; ++c) {
                             uint32_t t[32];
                             tmem_ld_x32(o_tmem + c * 32, t);
@@ -925,8 +933,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                         t[i] = pack_bf16x2(p0.x, p0.y);
                         t[i + 1] = pack_bf16x2(p1.x, p1.y);
                     }
-                    tmem_st_x32(s_tmem + c * 32, t);
+                    if (c == 0 && pv_pending) {
+                        ok = wait_pv();
+                        if (!ok) break;
+                    }
+                    tmem_st_x32(p_tmem + c * 32, t);
                 }
+                if (!ok) break;
                 l += (acc0.x + acc0.y) + (acc1.x + acc1.y);
                 PH_MARK(4);
                 tmem_wait_st();
@@ -939,9 +952,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             float inv = 0.f;
             float lse_val = -INFINITY;
             if (nblk > 0) {
-                ok = mbar_wait(wctx, smem_u32(&sh.o_full[x]), o_cnt & 1u, 12);
+                ok = mbar_wait(wctx, smem_u32(&sh.pv_done[x]), pv_cnt & 1u, 12);
                 if (!ok) break;
-                ++o_cnt;
+                ++pv_cnt;
                 tc_fence_after_sync();
                 // A row that never saw a key keeps m_used = -inf (its polynomial exponentials are
                 // 2^-126 rather than exactly 0, so the row sum alone does not tell).
@@ -1065,7 +1078,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     // Common exit: every role arrives here (normally or after an abort).
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == kFwdMmaWarp) {
+    if (warp == kFwdQkWarp) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 512);
     }
