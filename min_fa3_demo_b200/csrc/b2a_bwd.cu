@@ -310,7 +310,6 @@ int b2a_bwd_with_scratch(const b2a_bwd_args* a, void* scratch, size_t scratch_by
         a->softmax_scale > 0.f ? a->softmax_scale : 1.0f / std::sqrt(static_cast<float>(kHeadDim));
     const int causal = a->is_causal ? 1 : 0;
 
-    B2A_CUDA_OK(cudaMemsetAsync(hdr, 0, sizeof(WorkspaceHeader), stream));
     int* dq_sem = nullptr;
     if (a->deterministic) {
         dq_sem = reinterpret_cast<int*>(ws + lay.dq_sem_off);
@@ -325,6 +324,7 @@ int b2a_bwd_with_scratch(const b2a_bwd_args* a, void* scratch, size_t scratch_by
     pre.lse = a->lse;
     pre.lse2 = lse2;
     pre.dpsum = dpsum;
+    pre.header = varlen ? nullptr : reinterpret_cast<int4*>(hdr);   // packed documents: the planner writes it
     pre.dq_accum = dq_accum;     // cleared by the preprocess: no separate memset pass
     pre.cu_seqlens_q = a->cu_seqlens_q;
     pre.batch = a->batch;
@@ -376,7 +376,7 @@ int b2a_bwd_with_scratch(const b2a_bwd_args* a, void* scratch, size_t scratch_by
     long long work_items;
     if (varlen) {
         rc = launch_varlen_plan(1, a->cu_seqlens_q, a->cu_seqlens_k, a->batch, causal, work_list,
-                                &hdr->num_entries, lay.entries_cap, stream);
+                                hdr, lay.entries_cap, stream);
         if (rc != B2A_OK) return rc;
         p.num_entries_host = lay.entries_cap;
         work_items = static_cast<long long>(lay.entries_cap) * a->heads_k;

@@ -1178,6 +1178,7 @@ struct BwdPreParams {
     const float* lse;
     float* lse2;
     float* dpsum;
+    int4* header;        // workspace header, zeroed here; may be null
     float* dq_accum;     // zeroed here (each CTA clears the 16 KiB slab matching its 32 rows); may be null
     const int* cu_seqlens_q;
     int batch;
@@ -1205,6 +1206,7 @@ bwd_preprocess_kernel(const BwdPreParams p) {
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int prow_base = blockIdx.x * kPreRows;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && p.header != nullptr) *p.header = make_int4(0, 0, 0, 0);
 
     if (threadIdx.x < kPreRows) {
         const int prow = prow_base + threadIdx.x;

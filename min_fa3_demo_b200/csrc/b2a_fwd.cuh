@@ -80,7 +80,7 @@ struct FwdParams {
     const int* cu_seqlens_k;
     const int2* work_list;       // varlen: (doc, m_block) in LPT order; null for BSHD
     const int* num_entries_dev;  // varlen: number of work_list entries (device word)
-    int* sched_counter;          // zeroed before launch
+    int* sched_counter;          // zeroed before launch; null: CTA i takes item i and no other
     unsigned int* status;
     int batch;
     int seqlen_q;                // BSHD: S_q.  varlen: unused
@@ -532,6 +532,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             mbar_init(smem_u32(&sh.comm_empty[i]), 1);
         }
         sh.abort_flag = 0;
+        // All CTAs of such a launch start together, long before any wait can run out.
+        if (p.sched_counter == nullptr && blockIdx.x == 0 && p.status != nullptr) *p.status = 0u;
         fence_mbar_init();
         fence_proxy_async_smem();
     }
@@ -575,8 +577,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             // Ring mode: true once all copy CTAs are done, i.e. every remote block has landed.
             bool all_landed = p.ring_docs == nullptr || p.comm_task_count == 0;
             const int copy_ctas = static_cast<int>(gridDim.x) - p.num_comp;
-            int ticket = 0;
-            if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);
+            const bool one_each = p.sched_counter == nullptr;
+            int ticket = static_cast<int>(blockIdx.x);
+            auto take = [&]() {
+                if (lane == 0) ticket = one_each ? total_work : atomicAdd(p.sched_counter, 1);
+            };
+            if (!one_each) take();
             for (uint32_t it = 0; ok; ++it) {
                 const uint32_t slot = it % kFwdSlots;
                 ok = mbar_wait(wctx, smem_u32(&sh.sched_empty[slot]), ((it / kFwdSlots) & 1u) ^ 1u, 1);
@@ -586,7 +592,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 while (true) {
                     wk = fwd_decode_work<kMode == kFwdSplit>(p, __shfl_sync(0xFFFFFFFFu, ticket, 0), total_work);
                     if (!wk.valid || (wk.m0 < wk.q_len && !(wk.pair && (wk.head & 1)))) break;
-                    if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);   // an item without query rows
+                    take();   // an item without query rows
                 }
                 if (lane == 0) {
                     sh.work[slot] = wk;
@@ -658,7 +664,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 // long one, it would tie the next to this CTA for as long (10 documents of up to 4,961 tokens without a
                 // mask: 190 us against 157, with single passes from 154 to 179 as the last round falls, as it was without
                 // the ring).
-                if (lane == 0) ticket = atomicAdd(p.sched_counter, 1);
+                take();
             }
         } else if (warp == kFwdQkWarp || warp == kFwdPvWarp) {
             // ------------------------------------------------------------ MMA warps

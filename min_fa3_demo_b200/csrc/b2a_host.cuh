@@ -119,9 +119,9 @@ int configure_fwd_kernel(const DeviceInfo& dev, int mode);
 
 // Planner launch (b2a_plan.cu).  kind 0: forward items (256 query rows of a
 // document, cost = visible key blocks).  kind 1: backward items (128 key rows
-// of a document, cost = query tiles that see them).
+// of a document, cost = query tiles that see them).  Writes the whole workspace header.
 int launch_varlen_plan(int kind, const int* cu_seqlens_q, const int* cu_seqlens_k, int batch,
-                       int causal, int2* work_list, int* num_entries, int max_entries_cap,
+                       int causal, int2* work_list, WorkspaceHeader* header, int max_entries_cap,
                        cudaStream_t stream);
 
 // Optional per-thread kernel timing (b2a_profile_enable / b2a_profile_read).  The launchers

@@ -43,7 +43,7 @@ __device__ __forceinline__ int plan_cost(int kind, int causal, int q_len, int k_
 
 __global__ void __launch_bounds__(kPlanThreads)
 varlen_plan_kernel(int kind, const int* __restrict__ cu_q, const int* __restrict__ cu_k, int batch,
-                   int causal, int2* __restrict__ work_list, int* __restrict__ num_entries,
+                   int causal, int2* __restrict__ work_list, WorkspaceHeader* __restrict__ header,
                    int max_entries_cap) {
     __shared__ int bucket[kCostBuckets];
     __shared__ int warp_sum[32];
@@ -94,7 +94,7 @@ varlen_plan_kernel(int kind, const int* __restrict__ cu_q, const int* __restrict
         const int excl = warp_sum[wid] + incl - mine;
         bucket[c_hi] = excl;
         bucket[c_lo] = excl + n_hi;
-        if (t == 0) *num_entries = min(total, max_entries_cap);
+        if (t == 0) *header = WorkspaceHeader{0, min(total, max_entries_cap), 0u, 0};   // no memset of its own
     }
     __syncthreads();
 
@@ -116,10 +116,10 @@ varlen_plan_kernel(int kind, const int* __restrict__ cu_q, const int* __restrict
 }  // namespace
 
 int launch_varlen_plan(int kind, const int* cu_seqlens_q, const int* cu_seqlens_k, int batch,
-                       int causal, int2* work_list, int* num_entries, int max_entries_cap,
+                       int causal, int2* work_list, WorkspaceHeader* header, int max_entries_cap,
                        cudaStream_t stream) {
     varlen_plan_kernel<<<1, kPlanThreads, 0, stream>>>(kind, cu_seqlens_q, cu_seqlens_k, batch, causal,
-                                                      work_list, num_entries, max_entries_cap);
+                                                      work_list, header, max_entries_cap);
     B2A_CUDA_OK(cudaGetLastError());
     return B2A_OK;
 }
