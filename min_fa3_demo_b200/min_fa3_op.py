@@ -10,6 +10,7 @@ entry points still works (for CPU-side argument checks) but every compute call r
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import threading
 from typing import Optional, Tuple, Union
@@ -156,17 +157,45 @@ def _grad_output(provided: Optional[torch.Tensor], like: torch.Tensor, name: str
     return provided
 
 
+_SM100 = set()     # indices of the devices that have passed the check below; a device's capability does not change
+
+
 def _check_device_capability(device: torch.device, what: str) -> None:
     major, minor = torch.cuda.get_device_capability(device)
     _check(major == 10,
            f"{what} only supports Blackwell SM100. Current device capability is {major}.{minor}")
+    _SM100.add(device.index)
+
+
+# The entry points first ask in one expression whether everything is as it should be, and go through the checks above one by
+# one, which say what is wrong, only if not: some thirty calls and their message texts took about a third of the host's time
+# of a short call (1 x 128, 32 heads: 30 us a call, 17 with this, _on_device, _stream_ptr and one call that fills the arguments).
+def _is_bf16(t: torch.Tensor, dim: int, index: int) -> bool:
+    return (t.is_cuda and t.dtype is torch.bfloat16 and t.dim() == dim and t.is_contiguous() and t.get_device() == index
+            and t.size(-1) == 128)
+
+
+def _is_cu_seqlens(t: torch.Tensor, index: int) -> bool:
+    return t.is_cuda and t.dtype is torch.int32 and t.dim() == 1 and t.is_contiguous() and t.get_device() == index
 
 
 # --------------------------------------------------------------------------------------
 # C-ABI plumbing
 # --------------------------------------------------------------------------------------
+# torch's own function, and may go.
+_RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_HERE = contextlib.nullcontext()
+
+
 def _stream_ptr(device: torch.device) -> int:
+    if _RAW_STREAM is not None and device.index is not None:
+        return _RAW_STREAM(device.index)
     return torch.cuda.current_stream(device).cuda_stream
+
+
+def _on_device(device: torch.device):
+    """``torch.cuda.device``, which asks for and sets the device twice, only where another one is current."""
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
@@ -193,24 +222,16 @@ def _call_fwd(q, k, v, out, lse, *, cu_q, cu_k, batch, seqlen_q, seqlen_k, heads
     lib = _cabi.load()
     total_q = q.numel() // (heads_q * 128)
     total_k = k.numel() // (heads_k * 128)
-    args = _cabi.FwdArgs()
-    args.q, args.k, args.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
-    args.out, args.lse = out.data_ptr(), lse.data_ptr()
-    args.cu_seqlens_q, args.cu_seqlens_k = _ptr(cu_q), _ptr(cu_k)
-    args.batch, args.seqlen_q, args.seqlen_k = batch, seqlen_q, seqlen_k
-    args.total_q, args.total_k = total_q, total_k
-    args.heads_q, args.heads_k, args.head_dim = heads_q, heads_k, 128
-    args.is_causal = int(bool(is_causal))
-    args.merge_running = int(bool(merge_running))
-    args.grid_blocks = int(grid_blocks or 0)
-    args.softmax_scale = 0.0
+    args = _cabi.FwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), _ptr(cu_q), _ptr(cu_k),
+                         batch, seqlen_q, seqlen_k, total_q, total_k, heads_q, heads_k, 128, int(bool(is_causal)),
+                         int(bool(merge_running)), int(grid_blocks or 0), 0.0)
     if prefetch is not None:
         src_k, src_v, dst_k, dst_v, blocks = prefetch
         args.prefetch_src_k, args.prefetch_src_v = src_k, src_v
         args.prefetch_dst_k, args.prefetch_dst_v = dst_k.data_ptr(), dst_v.data_ptr()
         args.prefetch_bytes = dst_k.numel() * dst_k.element_size()
         args.prefetch_blocks = int(blocks)
-    with torch.cuda.device(q.device):
+    with _on_device(q.device):
         ref = ctypes.byref(args)
         nbytes = lib.b2a_fwd_scratch_bytes(ref) if may_cut else 0
         scratch = None
@@ -234,19 +255,10 @@ def _call_bwd(dout, q, k, v, out, lse, dq, dk, dv, *, cu_q, cu_k, batch, seqlen_
     lib = _cabi.load()
     total_q = q.numel() // (heads_q * 128)
     total_k = k.numel() // (heads_k * 128)
-    args = _cabi.BwdArgs()
-    args.dout, args.q, args.k, args.v = dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
-    args.out, args.lse = out.data_ptr(), lse.data_ptr()
-    args.dq, args.dk, args.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    args.cu_seqlens_q, args.cu_seqlens_k = _ptr(cu_q), _ptr(cu_k)
-    args.batch, args.seqlen_q, args.seqlen_k = batch, seqlen_q, seqlen_k
-    args.total_q, args.total_k = total_q, total_k
-    args.heads_q, args.heads_k, args.head_dim = heads_q, heads_k, 128
-    args.is_causal = int(bool(is_causal))
-    args.deterministic = int(bool(deterministic))
-    args.grid_blocks = 0
-    args.softmax_scale = 0.0
-    with torch.cuda.device(q.device):
+    args = _cabi.BwdArgs(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
+                         dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _ptr(cu_q), _ptr(cu_k), batch, seqlen_q, seqlen_k,
+                         total_q, total_k, heads_q, heads_k, 128, int(bool(is_causal)), int(bool(deterministic)), 0, 0.0)
+    with _on_device(q.device):
         ref = ctypes.byref(args)
         nbytes = lib.b2a_bwd_workspace_bytes(batch, total_q, total_k, heads_q, heads_k, 0 if cu_q is None else 1)
         more = lib.b2a_bwd_scratch_bytes(ref) - nbytes if may_cut and cu_q is None else 0
@@ -297,16 +309,7 @@ def check_last_status(entry_point: Optional[str] = None) -> None:
 # --------------------------------------------------------------------------------------
 # public API
 # --------------------------------------------------------------------------------------
-def forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: bool, *,
-            manual_block_count: Optional[int] = None, return_lse: bool = False
-            ) -> Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]]:
-    """BSHD attention forward (reference: ``forward``, bindings.cpp:240-278).
-
-    q ``[B, S, QH, 128]``, k/v ``[B, Sk, KVH, 128]`` bf16 contiguous; returns ``out`` like q and,
-    with ``return_lse``, the fp32 natural-log LSE ``[B, QH, S]``.  Repeated calls give the same bits;
-    the last bits can depend on how many sequences and heads share the call (``b2a_fwd_scratch_bytes``).
-    """
-    manual = _validate_manual_block_count(manual_block_count)
+def _check_forward(q, k, v) -> None:
     _check_bshd(q, "q")
     _check_bshd(k, "k")
     _check_bshd(v, "v")
@@ -321,29 +324,34 @@ def forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: bool, 
     _check(v.size(3) == 128, "v must have head_dim D=128")
     _check_device_capability(q.device, "min_fa3_demo_b200")
 
+
+def forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: bool, *,
+            manual_block_count: Optional[int] = None, return_lse: bool = False
+            ) -> Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]]:
+    """BSHD attention forward (reference: ``forward``, bindings.cpp:240-278).
+
+    q ``[B, S, QH, 128]``, k/v ``[B, Sk, KVH, 128]`` bf16 contiguous; returns ``out`` like q and,
+    with ``return_lse``, the fp32 natural-log LSE ``[B, QH, S]``.  Repeated calls give the same bits;
+    the last bits can depend on how many sequences and heads share the call (``b2a_fwd_scratch_bytes``).
+    """
+    manual = _validate_manual_block_count(manual_block_count)
+    index, qs, ks = q.get_device(), q.shape, k.shape
+    if not (_is_bf16(q, 4, index) and _is_bf16(k, 4, index) and _is_bf16(v, 4, index) and ks == v.shape and qs[0] == ks[0]
+            and qs[2] % ks[2] == 0 and index in _SM100):
+        _check_forward(q, k, v)
+
     out = torch.empty_like(q)
-    lse = torch.empty((q.size(0), q.size(2), q.size(1)), dtype=torch.float32, device=q.device)
-    ws = _call_fwd(q, k, v, out, lse, cu_q=None, cu_k=None, batch=q.size(0), seqlen_q=q.size(1),
-                   seqlen_k=k.size(1), heads_q=q.size(2), heads_k=k.size(2), is_causal=is_causal,
-                   grid_blocks=manual or 0)
+    lse = torch.empty((qs[0], qs[2], qs[1]), dtype=torch.float32, device=q.device)
+    ws = _call_fwd(q, k, v, out, lse, cu_q=None, cu_k=None, batch=qs[0], seqlen_q=qs[1], seqlen_k=ks[1], heads_q=qs[2],
+                   heads_k=ks[2], is_causal=is_causal, grid_blocks=manual or 0)
     _remember_workspace("forward", ws)
     if return_lse:
         return out, lse
     return out
 
 
-def forward_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
-                   cu_seqlens_q: torch.Tensor, cu_seqlens_k: torch.Tensor,
-                   max_seqlen_q: int, max_seqlen_k: int, is_causal: bool, *,
-                   cu_seqlens_q_host: torch.Tensor, cu_seqlens_k_host: torch.Tensor,
-                   manual_block_count: Optional[int] = None, return_lse: bool = False
-                   ) -> Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]]:
-    """Packed varlen attention forward (reference: ``forward_varlen``, bindings.cpp:280-363).
-
-    q ``[total_q, QH, 128]``, k/v ``[total_k, KVH, 128]``; LSE layout ``[QH, total_q]``.
-    """
-    manual = _validate_manual_block_count(manual_block_count)
-    max_seqlen_q, max_seqlen_k = int(max_seqlen_q), int(max_seqlen_k)
+def _check_forward_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, cu_seqlens_q_host,
+                          cu_seqlens_k_host) -> None:
     _check_varlen_qkv(q, "q")
     _check_varlen_qkv(k, "k")
     _check_varlen_qkv(v, "v")
@@ -365,16 +373,39 @@ def forward_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     _check(max_seqlen_q <= _INT32_MAX and max_seqlen_k <= _INT32_MAX, "max seqlens must fit in int32")
     _check_device_capability(q.device, "min_fa3_demo_b200")
 
+
+def forward_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
+                   cu_seqlens_q: torch.Tensor, cu_seqlens_k: torch.Tensor,
+                   max_seqlen_q: int, max_seqlen_k: int, is_causal: bool, *,
+                   cu_seqlens_q_host: torch.Tensor, cu_seqlens_k_host: torch.Tensor,
+                   manual_block_count: Optional[int] = None, return_lse: bool = False
+                   ) -> Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]]:
+    """Packed varlen attention forward (reference: ``forward_varlen``, bindings.cpp:280-363).
+
+    q ``[total_q, QH, 128]``, k/v ``[total_k, KVH, 128]``; LSE layout ``[QH, total_q]``.
+    """
+    manual = _validate_manual_block_count(manual_block_count)
+    max_seqlen_q, max_seqlen_k = int(max_seqlen_q), int(max_seqlen_k)
+    index, qs, ks = q.get_device(), q.shape, k.shape
+    if not (_is_bf16(q, 3, index) and _is_bf16(k, 3, index) and _is_bf16(v, 3, index) and _is_cu_seqlens(cu_seqlens_q, index)
+            and _is_cu_seqlens(cu_seqlens_k, index) and ks[1] == v.size(1) and qs[1] % ks[1] == 0
+            and cu_seqlens_k.numel() == cu_seqlens_q.numel() >= 2
+            and all(not t.is_cuda and t.dtype is torch.int32 and t.dim() == 1 and t.is_contiguous()
+                    and t.numel() == cu_seqlens_q.numel() for t in (cu_seqlens_q_host, cu_seqlens_k_host))
+            and 0 < max_seqlen_q <= _INT32_MAX and 0 < max_seqlen_k <= _INT32_MAX and index in _SM100):
+        _check_forward_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, cu_seqlens_q_host,
+                              cu_seqlens_k_host)
+
     batch = cu_seqlens_q_host.size(0) - 1
     _check(batch >= 1, "varlen demo requires batch size B >= 1")
-    _check(int(cu_seqlens_q_host[0]) == 0, "cu_seqlens_q_host must start with 0")
-    _check(int(cu_seqlens_k_host[0]) == 0, "cu_seqlens_k_host must start with 0")
-    _check(int(cu_seqlens_q_host[batch]) == q.size(0),
-           f"cu_seqlens_q_host[-1] must equal q.size(0). Got {int(cu_seqlens_q_host[batch])} "
-           f"vs {q.size(0)}")
-    _check(int(cu_seqlens_k_host[batch]) == k.size(0),
-           f"cu_seqlens_k_host[-1] must equal k.size(0). Got {int(cu_seqlens_k_host[batch])} "
-           f"vs {k.size(0)}")
+    first_q, last_q = cu_seqlens_q_host[::batch].tolist()
+    first_k, last_k = (first_q, last_q) if cu_seqlens_k_host is cu_seqlens_q_host else cu_seqlens_k_host[::batch].tolist()
+    _check(first_q == 0, "cu_seqlens_q_host must start with 0")
+    _check(first_k == 0, "cu_seqlens_k_host must start with 0")
+    if last_q != qs[0]:
+        raise RuntimeError(f"cu_seqlens_q_host[-1] must equal q.size(0). Got {last_q} vs {qs[0]}")
+    if last_k != ks[0]:
+        raise RuntimeError(f"cu_seqlens_k_host[-1] must equal k.size(0). Got {last_k} vs {ks[0]}")
 
     out = torch.empty_like(q)
     lse = torch.empty((q.size(1), q.size(0)), dtype=torch.float32, device=q.device)
@@ -387,17 +418,7 @@ def forward_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     return out
 
 
-def backward(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
-             out: torch.Tensor, softmax_lse: torch.Tensor, is_causal: bool, *,
-             deterministic: bool = False, dq: Optional[torch.Tensor] = None,
-             dk: Optional[torch.Tensor] = None, dv: Optional[torch.Tensor] = None
-             ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    """BSHD attention backward (reference: ``backward``, min_fa3_bwd_bindings.cu:156-253).
-
-    Returns ``(dq, dk, dv)``; caller-provided buffers are written in place and returned.  dk and dv
-    (and dq with ``deterministic``) repeat bit for bit; their last bits can depend on how many
-    sequences and heads share the call (``b2a_bwd_scratch_bytes``).
-    """
+def _check_backward(dout, q, k, v, out, softmax_lse) -> None:
     _check_bf16_cuda(q, "q", 4)
     _check_bf16_cuda(k, "k", 4)
     _check_bf16_cuda(v, "v", 4)
@@ -418,6 +439,26 @@ def backward(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
     _check(tuple(softmax_lse.shape) == (q.size(0), q.size(2), q.size(1)),
            "softmax_lse must have shape [B, QH, Sq]")
     _check_device_capability(q.device, "min_fa3_demo_b200 backward")
+
+
+def backward(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
+             out: torch.Tensor, softmax_lse: torch.Tensor, is_causal: bool, *,
+             deterministic: bool = False, dq: Optional[torch.Tensor] = None,
+             dk: Optional[torch.Tensor] = None, dv: Optional[torch.Tensor] = None
+             ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """BSHD attention backward (reference: ``backward``, min_fa3_bwd_bindings.cu:156-253).
+
+    Returns ``(dq, dk, dv)``; caller-provided buffers are written in place and returned.  dk and dv
+    (and dq with ``deterministic``) repeat bit for bit; their last bits can depend on how many
+    sequences and heads share the call (``b2a_bwd_scratch_bytes``).
+    """
+    index, qs, ks = q.get_device(), q.shape, k.shape
+    if not (_is_bf16(q, 4, index) and _is_bf16(k, 4, index) and _is_bf16(v, 4, index) and _is_bf16(out, 4, index)
+            and _is_bf16(dout, 4, index) and softmax_lse.is_cuda and softmax_lse.dtype is torch.float32
+            and softmax_lse.is_contiguous() and softmax_lse.get_device() == index and qs[0] > 0 and qs[1] > 0 and ks[1] > 0
+            and qs[0] == ks[0] and ks == v.shape and qs[2] % ks[2] == 0 and out.shape == qs and dout.shape == qs
+            and softmax_lse.shape == (qs[0], qs[2], qs[1]) and index in _SM100):
+        _check_backward(dout, q, k, v, out, softmax_lse)
     dq = _grad_output(dq, q, "dq")
     dk = _grad_output(dk, k, "dk")
     dv = _grad_output(dv, v, "dv")
@@ -428,15 +469,8 @@ def backward(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
     return dq, dk, dv
 
 
-def backward_varlen(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
-                    out: torch.Tensor, softmax_lse: torch.Tensor, cu_seqlens_q: torch.Tensor,
-                    cu_seqlens_k: torch.Tensor, max_seqlen_q: int, max_seqlen_k: int,
-                    is_causal: bool, *, deterministic: bool = False,
-                    dq: Optional[torch.Tensor] = None, dk: Optional[torch.Tensor] = None,
-                    dv: Optional[torch.Tensor] = None
-                    ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    """Packed varlen backward (reference: ``backward_varlen``, min_fa3_bwd_bindings.cu:255-357)."""
-    max_seqlen_q, max_seqlen_k = int(max_seqlen_q), int(max_seqlen_k)
+def _check_backward_varlen(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q,
+                           max_seqlen_k) -> None:
     _check_bf16_cuda(q, "q", 3)
     _check_bf16_cuda(k, "k", 3)
     _check_bf16_cuda(v, "v", 3)
@@ -462,6 +496,26 @@ def backward_varlen(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: tor
     _check(tuple(softmax_lse.shape) == (q.size(1), q.size(0)),
            "softmax_lse must have shape [QH, total_q]")
     _check_device_capability(q.device, "min_fa3_demo_b200 backward")
+
+
+def backward_varlen(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
+                    out: torch.Tensor, softmax_lse: torch.Tensor, cu_seqlens_q: torch.Tensor,
+                    cu_seqlens_k: torch.Tensor, max_seqlen_q: int, max_seqlen_k: int,
+                    is_causal: bool, *, deterministic: bool = False,
+                    dq: Optional[torch.Tensor] = None, dk: Optional[torch.Tensor] = None,
+                    dv: Optional[torch.Tensor] = None
+                    ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """Packed varlen backward (reference: ``backward_varlen``, min_fa3_bwd_bindings.cu:255-357)."""
+    max_seqlen_q, max_seqlen_k = int(max_seqlen_q), int(max_seqlen_k)
+    index, qs, ks = q.get_device(), q.shape, k.shape
+    if not (_is_bf16(q, 3, index) and _is_bf16(k, 3, index) and _is_bf16(v, 3, index) and _is_bf16(out, 3, index)
+            and _is_bf16(dout, 3, index) and softmax_lse.is_cuda and softmax_lse.dtype is torch.float32
+            and softmax_lse.is_contiguous() and softmax_lse.get_device() == index and _is_cu_seqlens(cu_seqlens_q, index)
+            and _is_cu_seqlens(cu_seqlens_k, index) and cu_seqlens_k.numel() == cu_seqlens_q.numel() >= 2 and qs[0] > 0
+            and ks[0] > 0 and ks == v.shape and qs[1] % ks[1] == 0 and out.shape == qs and dout.shape == qs
+            and 0 < max_seqlen_q <= _INT32_MAX and 0 < max_seqlen_k <= _INT32_MAX and softmax_lse.shape == (qs[1], qs[0])
+            and index in _SM100):
+        _check_backward_varlen(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k)
     dq = _grad_output(dq, q, "dq")
     dk = _grad_output(dk, k, "dk")
     dv = _grad_output(dv, v, "dv")

@@ -299,3 +299,35 @@ def test_calls_with_an_item_for_each_cta(b, s, qh, kvh):
         out2, lse2 = min_fa3_op.forward(q, k, v, causal, return_lse=True, manual_block_count=1)
         min_fa3_op_impl.check_last_status("forward")
         assert torch.equal(out, out2) and torch.equal(lse, lse2)
+
+
+@pytest.mark.parametrize("change", ["dtype", "rank", "width", "strides", "cpu", "batch", "keys", "kv_heads", "group"])
+def test_refusals_after_a_good_call(change):
+    """Once a device is known, the checks are one expression: it has to send every bad call to the one that says why."""
+    q, k, v = (torch.randn(2, 128, h, 128, device="cuda", dtype=torch.bfloat16) for h in (4, 2, 2))
+    out, lse = min_fa3_op.forward(q, k, v, True, return_lse=True)
+    min_fa3_op.backward(out, q, k, v, out, lse, True)
+    bad = {"dtype": lambda: k.half(), "rank": lambda: k[0], "width": lambda: k[..., :64].contiguous(),
+           "strides": lambda: k.transpose(1, 2).contiguous().transpose(1, 2), "cpu": lambda: k.cpu(),
+           "batch": lambda: k[:1].contiguous(), "keys": lambda: k[:, :64].contiguous(), "kv_heads": lambda: k[:, :, :1].contiguous(),
+           "group": lambda: torch.cat([k, k[:, :, :1]], 2)}[change]()
+    with pytest.raises(RuntimeError):
+        min_fa3_op.forward(q, bad, torch.cat([v, v[:, :, :1]], 2) if change == "group" else v, True)
+    with pytest.raises(RuntimeError):
+        min_fa3_op.backward(out, q, bad, torch.cat([v, v[:, :, :1]], 2) if change == "group" else v, out, lse, True)
+    cu = torch.tensor([0, 128, 256], dtype=torch.int32)
+    qp, kp, vp = (t.flatten(0, 1) for t in (q, k, v))
+    o, l = min_fa3_op.forward_varlen(qp, kp, vp, cu.cuda(), cu.cuda(), 128, 128, True, cu_seqlens_q_host=cu, cu_seqlens_k_host=cu,
+                                     return_lse=True)
+    if change in ("dtype", "width", "strides", "cpu", "kv_heads", "group", "rank"):
+        bad = {"rank": kp[0], "strides": kp.transpose(0, 1).contiguous().transpose(0, 1)}.get(change, bad.flatten(0, 1))
+        vg = torch.cat([vp, vp[:, :1]], 1) if change == "group" else vp
+        with pytest.raises(RuntimeError):
+            min_fa3_op.forward_varlen(qp, bad, vg, cu.cuda(), cu.cuda(), 128, 128, True, cu_seqlens_q_host=cu,
+                                      cu_seqlens_k_host=cu)
+        with pytest.raises(RuntimeError):
+            min_fa3_op.backward_varlen(o, qp, bad, vg, o, l, cu.cuda(), cu.cuda(), 128, 128, True)
+    for host in (cu.long(), cu[:2], torch.tensor([1, 128, 256], dtype=torch.int32), torch.tensor([0, 128, 255], dtype=torch.int32)):
+        with pytest.raises(RuntimeError):
+            min_fa3_op.forward_varlen(qp, kp, vp, cu.cuda(), cu.cuda(), 128, 128, True, cu_seqlens_q_host=host,
+                                      cu_seqlens_k_host=cu)
