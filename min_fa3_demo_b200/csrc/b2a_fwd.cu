@@ -131,6 +131,8 @@ fwd_combine_kernel(const FwdParams p) {
     constexpr int kPitch = kHeadDim + 4;    // bf16; keeps the 8-byte column stores of 16 rows on distinct banks
     __shared__ __align__(8) __nv_bfloat16 out[kCombineRows * kPitch];
     __shared__ float weight[kFwdMaxSplits][kCombineRows];
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     const int strips = (p.split_rows + kCombineRows - 1) / kCombineRows;
     const int strip = blockIdx.x % strips;
     const int x = blockIdx.x / strips % p.split_tiles;
@@ -386,15 +388,15 @@ int b2a_fwd_with_scratch(const b2a_fwd_args* a, void* scratch, size_t scratch_by
     if (rc != B2A_OK) return rc;
     profile_mark(B2A_KERNEL_FWD, false, stream);
     if (mode == kFwdMerge) {
-        fwd_kernel<kFwdMerge><<<grid, kFwdThreads, kFwdSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        B2A_CUDA_OK(launch_early(fwd_kernel<kFwdMerge>, grid, kFwdThreads, kFwdSmemBytes, stream, map_q, map_k, map_v, p));
     } else if (mode == kFwdSplit) {
-        fwd_kernel<kFwdSplit><<<grid, kFwdThreads, kFwdSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        B2A_CUDA_OK(launch_early(fwd_kernel<kFwdSplit>, grid, kFwdThreads, kFwdSmemBytes, stream, map_q, map_k, map_v, p));
     } else {
-        fwd_kernel<kFwdPlain><<<grid, kFwdThreads, kFwdSmemBytes, stream>>>(map_q, map_k, map_v, p);
+        B2A_CUDA_OK(launch_early(fwd_kernel<kFwdPlain>, grid, kFwdThreads, kFwdSmemBytes, stream, map_q, map_k, map_v, p));
     }
     if (mode == kFwdSplit) {
         const long long strips = static_cast<long long>(split.items) * split.tiles * ((split.rows + kCombineRows - 1) / kCombineRows);
-        fwd_combine_kernel<<<static_cast<unsigned int>(strips), 256, 0, stream>>>(p);
+        B2A_CUDA_OK(launch_early(fwd_combine_kernel, static_cast<unsigned int>(strips), 256, 0, stream, p));
     }
     profile_mark(B2A_KERNEL_FWD, true, stream);
     B2A_CUDA_OK(cudaGetLastError());

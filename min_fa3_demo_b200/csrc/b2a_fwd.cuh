@@ -532,8 +532,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             mbar_init(smem_u32(&sh.comm_empty[i]), 1);
         }
         sh.abort_flag = 0;
-        // All CTAs of such a launch start together, long before any wait can run out.
-        if (p.sched_counter == nullptr && blockIdx.x == 0 && p.status != nullptr) *p.status = 0u;
         fence_mbar_init();
         fence_proxy_async_smem();
     }
@@ -542,6 +540,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
         tmem_relinquish();
         tc_fence_before_sync();
     }
+    let_next_kernel_start();
+    wait_for_previous_kernel();
+    // All CTAs of such a launch start together, long before any wait can run out.
+    if (p.sched_counter == nullptr && blockIdx.x == 0 && threadIdx.x == 0 && p.status != nullptr) *p.status = 0u;
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh.tmem_base);

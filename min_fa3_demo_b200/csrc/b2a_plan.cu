@@ -7,6 +7,7 @@
 //
 // One CTA plans the whole batch (a packed batch has at most a few thousand pieces).
 #include "b2a_host.cuh"
+#include "b2a_ptx.cuh"
 
 namespace b2a {
 
@@ -49,8 +50,10 @@ varlen_plan_kernel(int kind, const int* __restrict__ cu_q, const int* __restrict
     __shared__ int warp_sum[32];
     __shared__ int total;
     static_assert(kCostBuckets == 2 * kPlanThreads, "the scan gives every thread two buckets");
+    let_next_kernel_start();
     for (int i = threadIdx.x; i < kCostBuckets; i += kPlanThreads) bucket[i] = 0;
     if (threadIdx.x == 0) total = 0;
+    wait_for_previous_kernel();
     __syncthreads();
 
     // Histogram of piece costs.
@@ -118,9 +121,8 @@ varlen_plan_kernel(int kind, const int* __restrict__ cu_q, const int* __restrict
 int launch_varlen_plan(int kind, const int* cu_seqlens_q, const int* cu_seqlens_k, int batch,
                        int causal, int2* work_list, WorkspaceHeader* header, int max_entries_cap,
                        cudaStream_t stream) {
-    varlen_plan_kernel<<<1, kPlanThreads, 0, stream>>>(kind, cu_seqlens_q, cu_seqlens_k, batch, causal,
-                                                      work_list, header, max_entries_cap);
-    B2A_CUDA_OK(cudaGetLastError());
+    B2A_CUDA_OK(launch_early(varlen_plan_kernel, 1, kPlanThreads, 0, stream, kind, cu_seqlens_q, cu_seqlens_k, batch, causal,
+                             work_list, header, max_entries_cap));
     return B2A_OK;
 }
 

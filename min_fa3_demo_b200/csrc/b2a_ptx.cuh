@@ -801,6 +801,17 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return r;
 }
 
+// Programmatic dependent launch (see launch_early).  A kernel lets the next one of its stream start as soon as there is room,
+// and itself waits until the one before it is complete before it touches global memory.  Without such a launch neither does
+// anything.  Every thread of every CTA waits, so that a kernel is never complete before its predecessors are.
+__device__ __forceinline__ void let_next_kernel_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+__device__ __forceinline__ void wait_for_previous_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <uint32_t RegCount>
 __device__ __forceinline__ void reg_alloc() {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RegCount));

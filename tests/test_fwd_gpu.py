@@ -331,3 +331,28 @@ def test_refusals_after_a_good_call(change):
         with pytest.raises(RuntimeError):
             min_fa3_op.forward_varlen(qp, kp, vp, cu.cuda(), cu.cuda(), 128, 128, True, cu_seqlens_q_host=host,
                                       cu_seqlens_k_host=cu)
+
+
+@pytest.mark.parametrize("b,s,qh,kvh", [(1, 128, 8, 8), (2, 640, 16, 4), (8, 1024, 16, 4)])
+def test_calls_that_feed_each_other(b, s, qh, kvh):
+    """A forward's kernels come up while the one before them ends: each has to wait for what that one writes.  Ten calls whose
+    queries are the last one's output give the same bits with and without a pause between them, dense and packed in turn."""
+    q0, k, v = (torch.randn(b, s, h, 128, device="cuda", dtype=torch.bfloat16) for h in (qh, kvh, kvh))
+    cu = torch.arange(0, (b + 1) * s, s, dtype=torch.int32)
+    cu_dev = cu.cuda()
+
+    def chain(pause):
+        q = q0
+        for i in range(10):
+            if i % 2 == 0:
+                q = min_fa3_op.forward(q, k, v, True)
+            else:
+                q = min_fa3_op.forward_varlen(q.flatten(0, 1), k.flatten(0, 1), v.flatten(0, 1), cu_dev, cu_dev, s, s, True,
+                                              cu_seqlens_q_host=cu, cu_seqlens_k_host=cu).view(b, s, qh, 128)
+            if pause:
+                torch.cuda.synchronize()
+        return q
+
+    expected = chain(True)
+    for _ in range(3):
+        assert torch.equal(chain(False), expected)
