@@ -356,3 +356,17 @@ def test_calls_that_feed_each_other(b, s, qh, kvh):
     expected = chain(True)
     for _ in range(3):
         assert torch.equal(chain(False), expected)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("s", [384, 1024, 1500])
+def test_bshd_forward_with_a_growing_maximum(s, causal):
+    """Blocks are taken from the last key to the first, and here each has larger scores than the one before, so O is rescaled
+    at nearly every block: each time the P V before it has to be done, and no S or P may be lost."""
+    q, k, v, _ = make_bshd(5, 1, s, 4, 2)
+    k = (k.float() * torch.linspace(24, 1, s).view(1, s, 1, 1)).to(torch.bfloat16)
+    out, lse = run_bshd(q, k, v, causal)
+    ref_out, ref_lse = orc.bshd_forward(q, k, v, causal)
+    # LSE up to about 100: 1e-3 holds for values of a few units, so the same relative bound for these.
+    assert_within("O", out, ref_out, orc.bf16_attention_error(q, k, v, causal)["o"])
+    assert (lse.cpu() - ref_lse).abs().max() <= 1e-3 * max(1.0, ref_lse.abs().max().item() / 8)
