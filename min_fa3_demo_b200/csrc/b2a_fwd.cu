@@ -22,8 +22,8 @@ int set_fwd_smem_attribute() {
 // log2 of the query heads that share a tile's rows: all heads of a K/V head's group where their number is a power of
 // two that divides a tile (a TMA box of 128 / group rows of group heads is then one tile), none otherwise.  A tile of few
 // query rows is mostly padding without it, and K and V are streamed once per head or pair of heads instead of once: one
-// token for 16 sequences of 4,001, 32 over 8 heads, takes 58 us packed and 121 us not.  Full sequences take a little less
-// as well (4 x 2,048: 148 and 154 us, 1 x 32,768: 7,874 and 7,921 us), so there is no line between few and many rows.
+// token for 16 sequences of 4,001, 32 over 8 heads, takes 46 us packed and 120 us not.  Full sequences take as long or a little
+// less (4 x 2,048: 146 and 148 us, 1 x 32,768: 6,326 and 6,320 us), so there is no line between few and many rows.
 int fwd_pack_shift(int heads_q, int heads_k) {
     const int group = heads_q / heads_k;
     if ((group & (group - 1)) != 0 || group > kTileM) return 0;
@@ -43,16 +43,17 @@ struct FwdSplit {
 
 // An item (up to 256 packed query rows against all keys they see) is the smallest thing a CTA takes.  Where there are
 // few items, or they fill the CTAs unevenly, the keys are cut as well.  The cost of k pieces per item, in K/V blocks a
-// CTA goes through (about 1.7 us each), is the number of rounds times the piece, plus one block a round for starting and
+// CTA goes through (about 1.6 us each), is the number of rounds times the piece, plus one block a round for starting and
 // storing a piece, three for the launch that adds up, and the time that writing and reading the pieces takes (about
 // 4 TB/s: they stay in L2).  Where items differ a lot in length (a square causal call) the dynamic hand-out packs them,
 // and the bound is the mean load plus half a piece.  A cut has to promise a twentieth: the model knows no better.
 // That formula picks the number of pieces, but it holds half a piece against an uncut causal call too, whose shortest items
 // come last and fill the gaps.  So the call is then handed out item by item both ways (HandOut), and again the cut has
 // to promise a twentieth: 1 x 6,829 causal, 8 over 2 heads, is 116 us uncut and was 127 cut.
-// Measured (us, not cut / cut): 512 rows against 16,384 keys, 32 over 8 heads, two pieces: 220 / 130; 2 x 3,001 rows
-// without a mask, 32 heads, the last of six rounds cut: 318 / 302; one square causal call of 2 x 1,024, 16 over 4 heads,
-// which this leaves alone: 39 / 49.  Groups that are no power of two are not packed, and their pairs of heads are not cut.
+// Measured (us, not cut / cut): 512 rows against 16,384 keys, 32 over 8 heads, two pieces: 211 / 130; 128 rows against 32,768:
+// 385 / 75; 4 x 64 rows against 8,192: 107 / 48; 2 x 3,001 rows without a mask, 32 heads, the last of six rounds cut: 268 / 261;
+// 1 x 6,829 causal, 8 over 2 heads, and 16 x 1 row against 4,001, which this leaves alone: 103 and 46.  Groups that are no
+// power of two are not packed, and their pairs of heads are not cut.
 FwdSplit plan_fwd_split(const b2a_fwd_args& a, int ctas) {
     FwdSplit s;
     const int group = a.heads_q / a.heads_k;
