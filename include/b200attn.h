@@ -348,13 +348,14 @@ int b2a_ring_bwd(const b2a_ring_bwd_args* args, void* cuda_stream);
 /* ------------------------------------------------------------------------- */
 
 /*
- * Synchronises the stream and reads the status word that kernels launched with
- * this workspace wrote.  Returns B2A_OK, or B2A_ERR_DEVICE_STATUS with the
- * decoded status in b2a_last_error() (for example a bounded wait that ran out).
- * No counterpart in the reference, whose device-side waits are unbounded
- * (include/mega_ring_semaphore.cuh:69-80).  workspace == NULL reads the status
- * word of the scratch built into the library, i.e. of the last b2a_fwd_noalloc
- * call on the current device.
+ * Synchronises the stream and reads the status word (of a forward with an item for
+ * each CTA: the words, one for each CTA) that kernels launched with this workspace
+ * wrote.  Returns B2A_OK, or B2A_ERR_DEVICE_STATUS with the decoded status in
+ * b2a_last_error() (for example a bounded wait that ran out).  No counterpart in the
+ * reference, whose device-side waits are unbounded
+ * (include/mega_ring_semaphore.cuh:69-80).  workspace == NULL reads the status of the
+ * scratch built into the library, i.e. of the last b2a_fwd_noalloc call on the
+ * current device.
  */
 int b2a_check_status(const void* workspace, void* cuda_stream);
 

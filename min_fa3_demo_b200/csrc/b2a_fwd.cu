@@ -228,11 +228,9 @@ int configure_fwd_kernel(const DeviceInfo& dev, int mode) {
 extern "C" {
 
 size_t b2a_fwd_workspace_bytes(int32_t batch, int32_t total_q, int32_t is_varlen) {
-    size_t bytes = sizeof(b2a::WorkspaceHeader);
-    if (is_varlen) {
-        bytes += b2a::max_entries(batch, total_q, b2a::kFwdRowsPerWork) * sizeof(int2);
-    }
-    return b2a::align_up(bytes, 256);
+    const size_t behind = is_varlen ? b2a::max_entries(batch, total_q, b2a::kFwdRowsPerWork) * sizeof(int2)
+                                    : b2a::kFwdStatusWords * sizeof(unsigned int);
+    return b2a::align_up(sizeof(b2a::WorkspaceHeader) + behind, 256);
 }
 
 size_t b2a_fwd_scratch_bytes(const b2a_fwd_args* a) {
@@ -290,7 +288,9 @@ int b2a_fwd_with_scratch(const b2a_fwd_args* a, void* scratch, size_t scratch_by
                 "workspace must be a 16-byte aligned device pointer");
     B2A_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 0xF) == 0, "scratch must be 16-byte aligned");
     const size_t need = b2a_fwd_workspace_bytes(a->batch, a->total_q, varlen ? 1 : 0);
-    if (a->workspace_bytes < need) {
+    // A fixed-length call without room for a status word per CTA runs all the same, with the counter.
+    const size_t least = varlen ? need : align_up(sizeof(WorkspaceHeader), 256);
+    if (a->workspace_bytes < least) {
         return fail(B2A_ERR_WORKSPACE_TOO_SMALL, "workspace has %zu bytes, need %zu",
                     a->workspace_bytes, need);
     }
@@ -367,12 +367,18 @@ int b2a_fwd_with_scratch(const b2a_fwd_args* a, void* scratch, size_t scratch_by
     }
 
     int grid = a->grid_blocks > 0 ? a->grid_blocks : dev.sm_count;
-    if (work_items <= std::min(grid, dev.sm_count) && !varlen) p.sched_counter = nullptr;   // every CTA has its item
+    // Packed documents: the planner writes the header.  One item a CTA and a status word for each: the kernel does.  Else a memset,
+    // a launch more: 2 to 3 us of a call that takes 9 (1 x 128, 32 heads) to 60.
+    if (!varlen && work_items <= std::min(grid, dev.sm_count) && a->workspace_bytes >= need &&
+        work_items + (prefetch ? a->prefetch_blocks : 0) <= kFwdStatusWords) {
+        p.sched_counter = nullptr;
+        p.status = reinterpret_cast<unsigned int*>(hdr + 1);
+        p.status_step = 1u;
+    } else if (!varlen) {
+        B2A_CUDA_OK(cudaMemsetAsync(hdr, 0, sizeof(WorkspaceHeader), stream));
+    }
     if (work_items < grid) grid = static_cast<int>(work_items);
     if (grid < 1) grid = 1;
-    // Packed documents: the planner writes the header.  One item a CTA: the kernel does.  A memset is a launch more, 2 to 3
-    // us of a call that takes 13 (1 x 128, 32 heads) to 60.
-    if (!varlen && p.sched_counter != nullptr) B2A_CUDA_OK(cudaMemsetAsync(hdr, 0, sizeof(WorkspaceHeader), stream));
     p.num_comp = grid;
     if (prefetch) {
         // Copy CTAs ride in the same launch behind the compute CTAs; neither kind waits for the other.

@@ -81,7 +81,8 @@ struct FwdParams {
     const int2* work_list;       // varlen: (doc, m_block) in LPT order; null for BSHD
     const int* num_entries_dev;  // varlen: number of work_list entries (device word)
     int* sched_counter;          // zeroed before launch; null: CTA i takes item i and no other
-    unsigned int* status;
+    unsigned int* status;        // one word, zeroed before launch; without a counter one for each CTA, behind the header
+    uint32_t status_step;        // 1: one for each CTA (from here, not a register: computed in the kernel 1 x 512 against 16,384 took 1.4 % more)
     int batch;
     int seqlen_q;                // BSHD: S_q.  varlen: unused
     int seqlen_k;
@@ -379,7 +380,7 @@ __device__ __forceinline__ bool flag_wait(const WaitCtx& ctx, const int* flag, u
             if (ld_shared_volatile_u32(ctx.abort_smem) != 0u) return false;
             if (global_timer_lo() - start > ctx.timeout_ns) {
                 st_shared_volatile_u32(ctx.abort_smem, 1u);
-                set_status(ctx.status, kStatusTimeout, (tag << 12) | (blockIdx.x & 0xFFFu));
+                set_status(ctx.status_word(), kStatusTimeout, (tag << 12) | (blockIdx.x & 0xFFFu));
                 return false;
             }
             __nanosleep(100);
@@ -542,13 +543,19 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
     }
     let_next_kernel_start();
     wait_for_previous_kernel();
-    // All CTAs of such a launch start together, long before any wait can run out.
-    if (p.sched_counter == nullptr && blockIdx.x == 0 && threadIdx.x == 0 && p.status != nullptr) *p.status = 0u;
+    // Without a counter nothing ran before this kernel to clear the header, and CTAs may start in any order and at any time, so
+    // a word that one of them clears is not another's to report in: each clears and uses its own, and CTA 0 writes the header.
+    if (p.status_step != 0u && threadIdx.x == 0) {
+        p.status[blockIdx.x] = 0u;
+        if (blockIdx.x == 0) {
+            reinterpret_cast<int4*>(p.status)[-1] = make_int4(-static_cast<int>(gridDim.x), 0, 0, 0);
+        }
+    }
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh.tmem_base);
 
-    WaitCtx wctx{smem_u32(&sh.abort_flag), p.status, p.timeout_ns};
+    WaitCtx wctx{smem_u32(&sh.abort_flag), p.status, p.timeout_ns, p.status_step};
 
     // Copy CTAs (ring mode): pull the other ranks' K/V blocks into the local arena first, then
     // join the attention work queue like every other CTA.

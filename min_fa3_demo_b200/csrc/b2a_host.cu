@@ -210,11 +210,20 @@ int b2a_check_status(const void* workspace, void* cuda_stream) {
     WorkspaceHeader hdr{};
     B2A_CUDA_OK(cudaMemcpyAsync(&hdr, workspace, sizeof(hdr), cudaMemcpyDeviceToHost, stream));
     B2A_CUDA_OK(cudaStreamSynchronize(stream));
-    if (hdr.status != 0) {
-        unsigned code = hdr.status >> 24;
-        unsigned detail = hdr.status & 0xFFFFFFu;
+    unsigned status = hdr.status;
+    if (hdr.sched_counter < 0 && hdr.sched_counter >= -kFwdStatusWords) {   // one word for each CTA: the first that is set
+        unsigned words[kFwdStatusWords];
+        const int count = -hdr.sched_counter;
+        B2A_CUDA_OK(cudaMemcpyAsync(words, static_cast<const WorkspaceHeader*>(workspace) + 1, count * sizeof(unsigned),
+                                    cudaMemcpyDeviceToHost, stream));
+        B2A_CUDA_OK(cudaStreamSynchronize(stream));
+        for (int i = 0; i < count && status == 0; ++i) status = words[i];
+    }
+    if (status != 0) {
+        unsigned code = status >> 24;
+        unsigned detail = status & 0xFFFFFFu;
         return fail(B2A_ERR_DEVICE_STATUS,
-                    "device status 0x%08x: %s (wait site %u, CTA %u)", hdr.status,
+                    "device status 0x%08x: %s (wait site %u, CTA %u)", status,
                     code == 1 ? "bounded wait timed out" : "device-side check failed",
                     detail >> 12, detail & 0xFFFu);
     }

@@ -51,7 +51,7 @@ int make_token_map(CUtensorMap* map, const void* base, uint64_t tokens, uint64_t
 
 // Header words at the start of every workspace.
 struct WorkspaceHeader {
-    int sched_counter;        // dynamic tile scheduler ticket
+    int sched_counter;        // dynamic tile scheduler ticket; -n: no tickets, and n status words, one for each CTA, behind the header
     int num_entries;          // varlen: number of planned work-list entries
     unsigned int status;      // device status word (0 = ok)
     int reserved;
@@ -78,6 +78,9 @@ cudaError_t launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_
     config.numAttrs = 1;
     return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
+
+// Room for such words in a fixed-length forward's workspace (a B200 has 148 SMs; the rest is for copy CTAs): 1 KiB with the header.
+constexpr int kFwdStatusWords = 252;
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

@@ -134,6 +134,9 @@ struct WaitCtx {
     uint32_t abort_smem;      // shared-memory address of the abort word
     unsigned int* status;     // in global memory (may be null)
     uint32_t timeout_ns;
+    uint32_t status_step;     // 0: one word for all CTAs, 1: CTA i has the i-th word from `status` on
+
+    __device__ __forceinline__ unsigned int* status_word() const { return status + status_step * blockIdx.x; }
 };
 
 // Bounded wait on an mbarrier phase.  `tag` identifies the wait site in the
@@ -156,7 +159,7 @@ __device__ __forceinline__ bool mbar_wait(const WaitCtx& ctx, uint32_t bar, uint
             }
             if (global_timer_lo() - start > ctx.timeout_ns) {
                 st_shared_volatile_u32(ctx.abort_smem, 1u);
-                set_status(ctx.status, kStatusTimeout, (tag << 12) | (blockIdx.x & 0xFFFu));
+                set_status(ctx.status_word(), kStatusTimeout, (tag << 12) | (blockIdx.x & 0xFFFu));
                 return false;
             }
         }

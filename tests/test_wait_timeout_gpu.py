@@ -1,4 +1,5 @@
-"""A bounded device-side wait that runs out, on one GPU, without faulting or hanging anything.
+"""A bounded device-side wait that runs out, on one GPU, without faulting or hanging anything, and the words that such a wait
+is reported in.
 
 Every spin wait of the kernels has a time limit; when it passes, the waiter records
 (wait site, CTA) in the workspace's status word and returns, and the host reads it with
@@ -11,6 +12,7 @@ usable, and the same call with a properly zeroed counter then succeeds.
 """
 from __future__ import annotations
 
+import ctypes
 import time
 
 import pytest
@@ -89,3 +91,41 @@ def test_completion_wait_runs_out_and_reports_status():
     assert_within("dQ", dq, rq, e["dq"])
     assert_within("dK", dk, rk_, e["dk"])
     assert_within("dV", dv, rv_, e["dv"])
+
+
+@pytest.mark.parametrize("b,s,qh,kvh", [(1, 130, 3, 3), (3, 70, 6, 1), (4, 256, 8, 8)])
+def test_each_cta_reports_in_a_word_of_its_own(b, s, qh, kvh):
+    """A call with an item for each CTA has nothing before its kernel that clears the workspace, so no CTA may report in a word
+    that another one clears: each has its own.  Starts from a workspace full of ones; an error is written into it by the test,
+    no wait runs out."""
+    lib = _cabi.load()
+    if torch.cuda.get_device_properties(0).multi_processor_count < 64:
+        pytest.skip("the cases need an SM for each item")
+    q, k, v = (torch.randn(b, s, h, 128, device="cuda", dtype=torch.bfloat16) for h in (qh, kvh, kvh))
+    out, lse = torch.empty_like(q), torch.empty(b, qh, s, device="cuda")
+    items = b * qh * ((s + 255) // 256)
+    need = lib.b2a_fwd_workspace_bytes(b, b * s, 0)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def call(nbytes):
+        ws = torch.full((need // 4,), -1, dtype=torch.int32, device="cuda")
+        a = _cabi.FwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), None, None, b, s, s, b * s,
+                          b * s, qh, kvh, 128, 1)
+        a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
+        _cabi.check(lib.b2a_fwd(ctypes.byref(a), stream))
+        assert lib.b2a_check_status(ws.data_ptr(), stream) == _cabi.B2A_OK, _cabi.last_error()
+        return ws, out.clone(), lse.clone()
+
+    ws, out1, lse1 = call(need)
+    words = ws.tolist()
+    assert words[0] == -items and words[4:4 + items] == [0] * items
+    assert all(w == -1 for w in words[4 + items:])
+    for cta in (0, items // 2, items - 1):
+        ws[4 + cta] = (1 << 24) | (9 << 12) | cta
+        assert lib.b2a_check_status(ws.data_ptr(), stream) == _cabi.B2A_ERR_DEVICE_STATUS
+        assert f"wait site 9, CTA {cta})" in _cabi.last_error()
+        ws[4 + cta] = 0
+    # Without room for the words, the counter and one word that a memset clears before the kernel.
+    ws, out2, lse2 = call(256)
+    assert ws.tolist()[0] > 0 and ws.tolist()[2] == 0 and all(w == -1 for w in ws.tolist()[4:])
+    assert torch.equal(out1, out2) and torch.equal(lse1, lse2)
