@@ -104,6 +104,11 @@ def _check_varlen_qkv(t: torch.Tensor, name: str) -> None:
     _check(t.is_contiguous(), f"{name} must be contiguous [total_tokens, H, D]")
 
 
+def _check_value_rows(k: torch.Tensor, v: torch.Tensor) -> None:
+    # V is read by k's token count; rows of v behind it are never looked at.
+    _check(k.size(0) <= v.size(0), f"v must not have fewer tokens than k. Got {v.size(0)} vs {k.size(0)}")
+
+
 def _check_cu_seqlens(t: torch.Tensor, name: str) -> None:
     _check(t.is_cuda, f"{name} must be a CUDA tensor")
     _check(t.dtype == torch.int32, f"{name} must have dtype torch.int32")
@@ -363,6 +368,7 @@ def _check_forward_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max
     _check(q.device == cu_seqlens_q.device and q.device == cu_seqlens_k.device,
            "q, k, v, cu_seqlens_q, and cu_seqlens_k must be on the same CUDA device")
     _check(k.size(1) == v.size(1), "k and v must have the same KV head count")
+    _check_value_rows(k, v)
     _check(q.size(1) % k.size(1) == 0,
            "This demo requires qhead % kvhead == 0 for GQA/MQA. "
            f"Got qhead={q.size(1)}, kvhead={k.size(1)}")
@@ -388,7 +394,7 @@ def forward_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     max_seqlen_q, max_seqlen_k = int(max_seqlen_q), int(max_seqlen_k)
     index, qs, ks = q.get_device(), q.shape, k.shape
     if not (_is_bf16(q, 3, index) and _is_bf16(k, 3, index) and _is_bf16(v, 3, index) and _is_cu_seqlens(cu_seqlens_q, index)
-            and _is_cu_seqlens(cu_seqlens_k, index) and ks[1] == v.size(1) and qs[1] % ks[1] == 0
+            and _is_cu_seqlens(cu_seqlens_k, index) and ks[1] == v.size(1) and ks[0] <= v.size(0) and qs[1] % ks[1] == 0
             and cu_seqlens_k.numel() == cu_seqlens_q.numel() >= 2
             and all(not t.is_cuda and t.dtype is torch.int32 and t.dim() == 1 and t.is_contiguous()
                     and t.numel() == cu_seqlens_q.numel() for t in (cu_seqlens_q_host, cu_seqlens_k_host))

@@ -18,7 +18,7 @@ import torch
 
 from . import _cabi
 from .min_fa3_op import (_INT32_MAX, _call_fwd, _check, _check_cu_seqlens, _check_cu_seqlens_host,
-                         _check_device_capability, _check_varlen_qkv, _remember_workspace, _stream_ptr,
+                         _check_device_capability, _check_value_rows, _check_varlen_qkv, _remember_workspace, _stream_ptr,
                          _workspace)
 from .parallel import TKParallelTensor
 
@@ -69,6 +69,7 @@ def _common_checks(q, k, v, cu_q, cu_k, cu_q_host, cu_k_host, max_q, max_k, num_
     _check(q.device == cu_q.device and q.device == cu_k.device,
            "q, k, v, cu_seqlens_q, and cu_seqlens_k must be on the same CUDA device")
     _check(k.size(1) == v.size(1), "k and v must have the same KV head count")
+    _check_value_rows(k, v)
     _check(q.size(1) % k.size(1) == 0,
            f"This demo requires qhead % kvhead == 0 for GQA/MQA. Got qhead={q.size(1)}, kvhead={k.size(1)}")
     _check(v.size(2) == 128, "v must have head_dim D=128")

@@ -5,9 +5,10 @@ from __future__ import annotations
 
 import pytest
 import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
 
 import min_fa3_op
-from min_fa3_demo_b200 import min_fa3_op as op
+from min_fa3_demo_b200 import min_fa3_op as op, ring
 
 
 def test_root_module_reexports_api():
@@ -68,3 +69,47 @@ def test_varlen_host_checks():
         op._check_cu_seqlens_host(torch.tensor([0, 8], dtype=torch.int32), cu_dev_like,
                                   "cu_seqlens_q_host")
     op._check_cu_seqlens_host(cu_dev_like.clone(), cu_dev_like, "cu_seqlens_q_host")
+
+
+# ---------------------------------------------------------------------------------------
+# Refusals of calls that are in order but for one argument.  The tensors are fakes on "cuda:0": sizes, types and strides, no
+# memory, so that nothing can be launched, here or on a GPU.
+# ---------------------------------------------------------------------------------------
+class Launched(Exception):
+    pass
+
+
+def on_cuda(*shape, dtype=torch.bfloat16, device="cuda:0"):
+    with FakeTensorMode():
+        return torch.empty(shape, dtype=dtype, device=device)
+
+
+@pytest.fixture(params=["device known", "device new"])
+def host_checks_only(request, monkeypatch):
+    """Both ways through the checks: the one expression first, and, on a device not seen before, the list at once."""
+    def launched(*args, **kwargs):
+        raise Launched
+
+    monkeypatch.setattr(op, "_SM100", {0} if request.param == "device known" else set())
+    monkeypatch.setattr(torch.cuda, "get_device_capability", lambda device=None: (10, 0))
+    for name in ("_call_fwd", "_call_bwd"):
+        monkeypatch.setattr(op, name, launched)
+
+
+def packed_arguments():
+    cu = torch.tensor([0, 100, 256], dtype=torch.int32)
+    return dict(q=on_cuda(256, 4, 128), k=on_cuda(256, 2, 128), v=on_cuda(256, 2, 128),
+                cu_seqlens_q=on_cuda(3, dtype=torch.int32), cu_seqlens_k=on_cuda(3, dtype=torch.int32), max_seqlen_q=156,
+                max_seqlen_k=156, is_causal=True, cu_seqlens_q_host=cu, cu_seqlens_k_host=cu)
+
+
+def test_packed_forward_refuses_fewer_values_than_keys(host_checks_only):
+    with pytest.raises(RuntimeError, match="v must not have fewer tokens than k. Got 255 vs 256"):
+        op.forward_varlen(**dict(packed_arguments(), v=on_cuda(255, 2, 128)))
+
+
+def test_context_parallel_forward_refuses_fewer_values_than_keys():
+    a = packed_arguments()
+    with pytest.raises(RuntimeError, match="v must not have fewer tokens than k. Got 255 vs 256"):
+        ring._common_checks(a["q"], a["k"], on_cuda(255, 2, 128), a["cu_seqlens_q"], a["cu_seqlens_k"], a["cu_seqlens_q_host"],
+                            a["cu_seqlens_k_host"], 156, 156, 1, 0)
