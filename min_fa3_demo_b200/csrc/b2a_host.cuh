@@ -59,7 +59,9 @@ struct WorkspaceHeader {
 static_assert(sizeof(WorkspaceHeader) == 16, "workspace header is 16 bytes");
 
 // Launches a kernel that begins with wait_for_previous_kernel (after what needs no global memory): its CTAs may come up while
-// the stream's previous kernel ends, which takes the launch, barriers, tensor memory and descriptors off the path.  Used by the
+// the stream's previous kernel ends, which takes the launch, barriers, tensor memory and descriptors off the path.  Such a
+// kernel lives while that one still writes, so no pointer of it is __restrict__ const and nothing is read through the
+// read-only path: both promise that the data does not change while the kernel lives.  Used by the
 // forward's kernels and the planner (us, without / with: 1 x 128, 32 heads 10.6 / 9.2; 16,384 tokens in short documents, two
 // kernels, 78.6 / 75.7; one token for 16 x 4,001 46.7 / 45.4; 512 rows against 16,384 keys, two kernels, 128.7 / 126.6), not by
 // the backward's: its CTAs then start one by one as the preprocess ends and stay out of step (4 x 8,192 causal 4,995 / 5,119;

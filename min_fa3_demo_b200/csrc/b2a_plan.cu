@@ -43,9 +43,8 @@ __device__ __forceinline__ int plan_cost(int kind, int causal, int q_len, int k_
 }
 
 __global__ void __launch_bounds__(kPlanThreads)
-varlen_plan_kernel(int kind, const int* __restrict__ cu_q, const int* __restrict__ cu_k, int batch,
-                   int causal, int2* __restrict__ work_list, WorkspaceHeader* __restrict__ header,
-                   int max_entries_cap) {
+varlen_plan_kernel(int kind, const int* cu_q, const int* cu_k, int batch, int causal, int2* work_list,
+                   WorkspaceHeader* header, int max_entries_cap) {
     __shared__ int bucket[kCostBuckets];
     __shared__ int warp_sum[32];
     __shared__ int total;

@@ -92,3 +92,15 @@ def test_workspace_sizes(lib):
     # backward: fp32 dQ accumulator dominates (heads_q * padded rows * 128 floats)
     bwd = lib.b2a_bwd_workspace_bytes(4, 4 * 8192, 4 * 8192, 32, 8, 0)
     assert bwd >= 32 * 4 * 8192 * 128 * 4
+
+
+def test_kernels_that_start_early_use_ordinary_loads():
+    # Read-only loads (a pointer declared __restrict__ const, __ldg, ld.global.nc) promise that what they read does not change
+    # while the kernel lives, and a kernel launched by launch_early lives while the one before it still writes.
+    source = "\n".join(p.read_text() for p in sorted(build.CSRC_DIR.glob("*.cu*")))
+    names = set(re.findall(r"launch_early\((\w+_kernel)\b", source))
+    assert names == {"fwd_kernel", "fwd_combine_kernel", "varlen_plan_kernel"}
+    for name in names:
+        signature = re.search(rf"__global__[^;{{]*?\b{name}\(([^{{]*?)\)\s*{{", source).group(1)
+        assert "__restrict__" not in signature, name
+    assert not re.search(r"__ldg\b|ld\.global\.nc", source)
