@@ -44,16 +44,17 @@ struct FwdSplit {
 // An item (up to 256 packed query rows against all keys they see) is the smallest thing a CTA takes.  Where there are
 // few items, or they fill the CTAs unevenly, the keys are cut as well.  The cost of k pieces per item, in K/V blocks a
 // CTA goes through (about 1.6 us each), is the number of rounds times the piece, plus one block a round for starting and
-// storing a piece, three for the launch that adds up, and the time that writing and reading the pieces takes (about
-// 4 TB/s: they stay in L2).  Where items differ a lot in length (a square causal call) the dynamic hand-out packs them,
+// storing a piece, three for the launch that adds up, and the time that writing and reading the pieces takes (6.8 MB in a
+// block's time, about 4.2 TB/s: they stay in L2).  Where items differ a lot in length (a square causal call) the dynamic hand-out packs them,
 // and the bound is the mean load plus half a piece.  A cut has to promise a twentieth: the model knows no better.
 // That formula picks the number of pieces, but it holds half a piece against an uncut causal call too, whose shortest items
 // come last and fill the gaps.  So the call is then handed out item by item both ways (HandOut), and again the cut has
-// to promise a twentieth: 1 x 6,829 causal, 8 over 2 heads, is 116 us uncut and was 127 cut.
-// Measured (us, not cut / cut): 512 rows against 16,384 keys, 32 over 8 heads, two pieces: 211 / 130; 128 rows against 32,768:
-// 385 / 75; 4 x 64 rows against 8,192: 107 / 48; 2 x 3,001 rows without a mask, 32 heads, the last of six rounds cut: 268 / 261;
-// 1 x 6,829 causal, 8 over 2 heads, and 16 x 1 row against 4,001, which this leaves alone: 103 and 46.  Groups that are no
-// power of two are not packed, and their pairs of heads are not cut.
+// to promise a twentieth.
+// Measured (us on the device, not cut / cut): 512 rows against 16,384 keys, 32 over 8 heads, two pieces: 194 / 114; 128 rows
+// against 32,768: 375 / 69; 4 x 64 rows against 8,192: 101 / 46; 2 x 3,001 rows without a mask, 32 heads, the last of six
+// rounds cut: 255 / 248.  Calls that this leaves alone, and what the formula's cut would make of them: 1 x 6,829 causal, 8 over
+// 2 heads, 91 / 101; 1 x 6,192, 8 over 1, 84 / 91; 2 x 1,024, 16 over 4, 21 / 35; 16 x 1 row against 4,001, 45 / 58.  Groups
+// that are no power of two are not packed, and their pairs of heads are not cut.
 FwdSplit plan_fwd_split(const b2a_fwd_args& a, int ctas) {
     FwdSplit s;
     const int group = a.heads_q / a.heads_k;

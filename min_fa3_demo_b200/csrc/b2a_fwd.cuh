@@ -18,18 +18,13 @@
 // A softmax warpgroup takes a whole row of S into registers, so the one S buffer serves both tiles in turn: while tile A
 // computes its probabilities, S of tile B is made, and the other way round.  P (bf16) has columns of its own and is consumed
 // by the P V MMA from tensor memory.  So neither Q K^T nor P V is on a tile's chain.  What bounds a pair of blocks is the
-// softmax of two warps per scheduler: about 2,650 clk against 2,048 of MMA (74 % of the tensor pipe; 3,200 and 62 % with S and
-// P of a tile in the same columns, where the chain was softmax -> P V -> Q K^T).  On long calls the clock gives a part of that
-// back (1.68 -> 1.59 GHz under the power cap): 8,192 keys, 32 over 8 heads: 852 -> 789 us, causal 454 -> 421; 4 x 2,048 causal
-// 152 -> 144; 512 rows against 16,384 keys 145 -> 132; one token for 16 x 4,001 60 -> 48.
+// softmax of two warps per scheduler: about 2,650 clk against 2,048 of MMA (74 % of the tensor pipe; 3,200 clk and 62 % if S and
+// P of a tile share columns: 8,192 keys, 32 over 8 heads, 789 against 852 us, causal 421 against 454).
 //   Q K^T and P V are issued by warps of their own: each instruction of an issuing warp waits its turn beside two dense
-// softmax warps, and one warp for both took 2,100 clk a tile and block for its waits and issues (8,192 causal: 516 us).
-// Leaving out the row maximum beyond an item's first block (the row sum tells when it is needed) was slower (443 against
-// 408 us): S then stays live through the exponentials.
+// softmax warps, and one warp for both needs 2,100 clk a tile and block for its waits and issues.
 //
 // Nothing stops between two work items: the load warp hands out decoded work items through a ring of kFwdSlots, and the next
-// item's first Q K^T only needs its Q and the S buffer.  A warpgroup of its own for the epilogue was slower: the softmax warps
-// then have 176 registers instead of 216 and spill (1,750 -> 1,840 us on 4 x 8,192).
+// item's first Q K^T only needs its Q and the S buffer.
 //
 // K and V tiles travel through two rings of 32 KiB stages, loaded in the order K(j) K(j-1) V(j) K(j-2) V(j-1) ...
 //
@@ -82,7 +77,8 @@ struct FwdParams {
     const int* num_entries_dev;  // varlen: number of work_list entries (device word)
     int* sched_counter;          // zeroed before launch; null: CTA i takes item i and no other
     unsigned int* status;        // one word, zeroed before launch; without a counter one for each CTA, behind the header
-    uint32_t status_step;        // 1: one for each CTA (from here, not a register: computed in the kernel 1 x 512 against 16,384 took 1.4 % more)
+    uint32_t status_step;        // 1: one for each CTA.  A parameter, because the waits have no register for it (1 x 512 rows
+                                 // against 16,384 keys 138.3 us with it computed in the kernel, 137.2 so)
     int batch;
     int seqlen_q;                // BSHD: S_q.  varlen: unused
     int seqlen_k;
@@ -671,8 +667,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                 if (!ok) break;
                 // The next ticket is taken no earlier than its K and V can be loaded: taken at the start of an item, a
                 // long one, it would tie the next to this CTA for as long (10 documents of up to 4,961 tokens without a
-                // mask: 190 us against 157, with single passes from 154 to 179 as the last round falls, as it was without
-                // the ring).
+                // mask: a fifth more time).
                 take();
             }
         } else if (warp == kFwdQkWarp || warp == kFwdPvWarp) {
@@ -790,8 +785,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
             ok = mbar_wait(wctx, smem_u32(&sh.sched_full[slot]), (it / kFwdSlots) & 1u, 10);
             if (!ok) break;
             // The slot is given back at the item's end: what only the epilogue needs is read again there instead of being
-            // kept in registers through the loop, where it made them spill (1 x 32,768 causal, 32 over 8 heads: 7,730 ->
-            // 7,660 us; 2 x 3,001 without a mask, 32 heads, cut: 315 -> 306).
+            // kept in registers through the loop, where it makes them spill (1 % of 1 x 32,768 causal, 32 over 8 heads, 3 % of
+            // 2 x 3,001 without a mask, 32 heads, cut).
             const FwdWork& wk = sh.work[slot];
             auto release = [&]() {
                 __syncwarp();
@@ -937,8 +932,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CU
                     for (int i = 0; i < 32; i += 2) {
                         const float2 x0 = fma2(make_float2(s[c * 64 + 2 * i], s[c * 64 + 2 * i + 1]), sl2v, negv);
                         const float2 x1 = fma2(make_float2(s[c * 64 + 2 * i + 2], s[c * 64 + 2 * i + 3]), sl2v, negv);
-                        // Half of the exponentials run on the special-function unit, half as a
-                        // polynomial on the FMA pipe, so the two units work side by side.
+                        // Where the mask has a bit, half of a group's exponentials run as a polynomial on the
+                        // FMA pipe (a quarter of all), beside the special-function unit's.
                         const float2 p0 = make_float2(fast_exp2(x0.x), fast_exp2(x0.y));
                         const float2 p1 = ((kFwdExpPolyMask >> (i / 2)) & 1u)
                                               ? exp2_poly2(x1)

@@ -115,13 +115,13 @@ def test_key_pieces_keep_nan_and_infinities(b, sq, sk, qh, kvh, causal):
 
 
 @pytest.mark.parametrize("cut,b,sq,sk,qh,kvh,causal", [
-    (True, 1, 512, 16384, 32, 8, True),      # 218 us uncut, 151 cut
-    (True, 2, 3001, 3001, 32, 32, False),    # 322 and 306: the last of six rounds
+    (True, 1, 512, 16384, 32, 8, True),      # 194 us uncut, 114 cut
+    (True, 2, 3001, 3001, 32, 32, False),    # 255 and 248: the last of six rounds
     (True, 1, 1, 4096, 8, 1, True),
     (False, 1, 1, 1024, 8, 1, True),         # eight blocks, and nothing gained
-    (False, 1, 6829, 6829, 8, 2, True),      # 116 and 127: the shortest items come last anyway
-    (False, 1, 6192, 6192, 8, 1, True),      # 93 and 100
-    (False, 2, 1024, 1024, 16, 4, True),     # 39 and 49
+    (False, 1, 6829, 6829, 8, 2, True),      # 91 and 101: the shortest items come last anyway
+    (False, 1, 6192, 6192, 8, 1, True),      # 84 and 91
+    (False, 2, 1024, 1024, 16, 4, True),     # 21 and 35
     (False, 1, 512, 16384, 24, 8, True),     # groups that are no power of two are not cut
 ])
 def test_which_calls_are_cut(cut, b, sq, sk, qh, kvh, causal):
