@@ -286,29 +286,39 @@ def test_full_size_rows_against_oracle_and_properties(causal):
     assert (out_ones.float() - 1.0).abs().max().item() <= 2.0 ** -7
 
 
-@pytest.mark.parametrize("b,s,qh,kvh", [(1, 1, 8, 2), (1, 130, 3, 3), (1, 128, 32, 32), (2, 1184, 16, 4), (2, 1185, 16, 4),
-                                        ("SMs - 1", 130, 1, 1), ("SMs", 130, 1, 1), ("SMs + 1", 130, 1, 1),
-                                        (3, 128, 6, 1), (1, 300, 6, 1)])
+@pytest.mark.parametrize("b,s,qh,kvh", [(1, 1, 8, 2), (1, 130, 3, 3), (1, 128, 32, 32), (2, 1184, 16, 4), (2, 1185, 16, 4)])
 def test_calls_with_an_item_for_each_cta(b, s, qh, kvh):
-    """At most as many items as SMs: nothing is handed out, and the kernel itself clears the status words.  One item a sequence
-    gives exactly as many items as SMs, one less and one more; the two cases of 1,184 and 1,185 rows have 152 items, and of 6
-    heads over 1 every second item of at most 128 rows is empty.  Fewer CTAs take the items from the counter instead; the
-    results are the same bits."""
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    b = {"SMs - 1": sms - 1, "SMs": sms, "SMs + 1": sms + 1}.get(b, b)
-    group = qh // kvh
-    packed = group & (group - 1) == 0
-    rows = 256 // group if packed else 256
-    items = b * ((s + rows - 1) // rows) * (kvh if packed else qh)
+    """The first three cases have at most as many items as CTAs: nothing is handed out, and the kernel itself clears the status
+    words (the last two have 152 items).  Fewer CTAs take the items from the counter instead; the results are the same bits."""
     q, k, v = (torch.randn(b, s, h, 128, device="cuda", dtype=torch.bfloat16) for h in (qh, kvh, kvh))
     for causal in (False, True):
-        dirty = [torch.full((n,), 255, dtype=torch.uint8, device="cuda") for n in (1024, 1024, 512)]
+        dirty = [torch.full((n,), 255, dtype=torch.uint8, device="cuda") for n in (256, 256, 512)]
         del dirty                                        # the workspace is likely to be one of these
         out, lse = min_fa3_op.forward(q, k, v, causal, return_lse=True)
         min_fa3_op_impl.check_last_status("forward")
-        if not is_cut("fwd", b, s, s, qh, kvh, causal):
-            ticket = min_fa3_op_impl._LAST.workspaces["forward"][:4].view(torch.int32).item()
-            assert ticket == -items if items <= sms else ticket > 0, "whether items were handed out"
+        out2, lse2 = min_fa3_op.forward(q, k, v, causal, return_lse=True, manual_block_count=1)
+        min_fa3_op_impl.check_last_status("forward")
+        assert torch.equal(out, out2) and torch.equal(lse, lse2)
+
+
+@pytest.mark.parametrize("b,s,qh,kvh", [(-1, 130, 1, 1), (0, 130, 1, 1), (1, 130, 1, 1), (3, 128, 6, 1), (1, 300, 6, 1)])
+def test_as_many_items_as_sms(b, s, qh, kvh):
+    """Exactly as many items as SMs, one less and one more (one key/value head: b counts from the number of SMs, a sequence is an
+    item), and calls of 6 heads over 1, of which every second item of at most 128 rows is empty.  The ticket in the workspace
+    says which way a call went; fewer CTAs, which take the items from the counter, give the same bits."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if qh == 1:
+        b += sms
+    items = b * ((s + 255) // 256) * qh                  # neither case packs heads into rows
+    q, k, v = (torch.randn(b, s, h, 128, device="cuda", dtype=torch.bfloat16) for h in (qh, kvh, kvh))
+    for causal in (False, True):
+        assert not is_cut("fwd", b, s, s, qh, kvh, causal)
+        dirty = [torch.full((n,), 255, dtype=torch.uint8, device="cuda") for n in (1024, 1024)]
+        del dirty                                        # the workspace is likely to be one of these
+        out, lse = min_fa3_op.forward(q, k, v, causal, return_lse=True)
+        min_fa3_op_impl.check_last_status("forward")
+        ticket = min_fa3_op_impl._LAST.workspaces["forward"][:4].view(torch.int32).item()
+        assert ticket == -items if items <= sms else ticket > 0, "whether items were handed out"
         out2, lse2 = min_fa3_op.forward(q, k, v, causal, return_lse=True, manual_block_count=1)
         min_fa3_op_impl.check_last_status("forward")
         assert torch.equal(out, out2) and torch.equal(lse, lse2)
